@@ -147,6 +147,26 @@ typedef struct spa_bwd_args {
 int spa_attn_bwd(const spa_bwd_args* args);
 
 /*
+ * The same forward and backward over the sequences of a packed batch (flash-attn's varlen
+ * layout), all of them in one launch per 32 sequences on the tensor-core path. The reference
+ * imports such functions without defining them (sp_aurora/adapters/hf_adapter.py:13-16,41-47).
+ *
+ * args: B = 1, Sq / Sk the packed token counts, no merge_prev / out_acc / dq_acc /
+ * dkv_accumulate, dq_overwrite set, dk / dv in the element type; causal_off is ignored.
+ * seqs: n sequences; sequence i has the query rows [q0, q0 + sq) and the key rows
+ * [k0, k0 + sk), both non-empty, in rising order and not overlapping, and its own causal
+ * offset. No sequence sees another one's rows. Rows of out, lse, dq, dk and dv that belong
+ * to no sequence are left as they are.
+ */
+typedef struct spa_seq {
+  int32_t q0, sq, k0, sk;
+  int32_t causal_off;
+} spa_seq;
+
+int spa_attn_varlen_fwd(const spa_fwd_args* args, const spa_seq* seqs, int32_t n);
+int spa_attn_varlen_bwd(const spa_bwd_args* args, const spa_seq* seqs, int32_t n);
+
+/*
  * Backward pass for callers that cannot allocate device memory.
  *
  * No counterpart in the reference. Who needs it: code that runs where every

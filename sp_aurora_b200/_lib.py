@@ -81,11 +81,19 @@ class BwdNoallocArgs(C.Structure):
     ]
 
 
+class Seq(C.Structure):
+    """One sequence of a packed batch (spa_seq)."""
+    _fields_ = [("q0", C.c_int32), ("sq", C.c_int32), ("k0", C.c_int32), ("sk", C.c_int32),
+                ("causal_off", C.c_int32)]
+
+
 # Every symbol include/spa.h declares, with its ctypes signature.
 _I64x4 = C.c_int64 * 4
 _SIGNATURES = {
     "spa_attn_fwd": (C.c_int, [C.POINTER(FwdArgs)]),
     "spa_attn_bwd": (C.c_int, [C.POINTER(BwdArgs)]),
+    "spa_attn_varlen_fwd": (C.c_int, [C.POINTER(FwdArgs), C.POINTER(Seq), C.c_int32]),
+    "spa_attn_varlen_bwd": (C.c_int, [C.POINTER(BwdArgs), C.POINTER(Seq), C.c_int32]),
     "spa_attn_bwd_noalloc": (C.c_int, [C.POINTER(BwdNoallocArgs)]),
     "spa_noalloc_scratch_bytes": (C.c_int64, []),
     "spa_bwd_delta": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
@@ -181,6 +189,11 @@ def device_info(device: int = 0) -> dict:
     check(lib.spa_device_info(device, buf), "spa_device_info")
     keys = ["sm_count", "cc_major", "cc_minor", "smem_optin_bytes", "l2_bytes", "global_mem_mib"]
     return dict(zip(keys, [int(x) for x in buf]))
+
+
+def seq_table(seqs):
+    """ctypes array of (q0, sq, k0, sk, causal_off) tuples for the spa_attn_varlen_* calls."""
+    return (Seq * len(seqs))(*seqs)
 
 
 def i64x4(vals):

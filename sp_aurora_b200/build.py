@@ -22,7 +22,7 @@ CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libspaurora_sm100.so"
 SOURCES = ["spa_abi.cu", "attn_fwd_sm100.cu", "attn_bwd_dq_sm100.cu", "attn_bwd_dkv_sm100.cu",
            "attn_simt.cu", "wait_selftest.cu"]
-HEADERS = [CSRC / "tc05.cuh", CSRC / "spa_internal.h", PKG_DIR.parent / "include" / "spa.h"]
+HEADERS = [CSRC / "tc05.cuh", CSRC / "varlen.cuh", CSRC / "spa_internal.h", PKG_DIR.parent / "include" / "spa.h"]
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",

@@ -37,6 +37,7 @@
 
 #include "spa_internal.h"
 #include "tc05.cuh"
+#include "varlen.cuh"
 
 namespace spa {
 namespace {
@@ -94,14 +95,18 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int D, typename T>
+// kVar: one launch over the sequences of a packed batch (B = 1, element-type dK/dV); Q and dO
+// are then read through the maps of the sequence's table entry, K and V through tm_k / tm_v
+// over the whole packed tensors.
+template <int D, typename T, bool kVar>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
                           const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v,
                           const __grid_constant__ CUtensorMap tm_do,
                           const __grid_constant__ CUtensorMap tm_dk,
-                          const __grid_constant__ CUtensorMap tm_dv, const DkvParams p) {
+                          const __grid_constant__ CUtensorMap tm_dv, const DkvParams p,
+                          const __grid_constant__ VarTable<kVar, 2> var) {
   using L = DkvSmem<D>;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   extern __shared__ uint8_t smem_raw[];
@@ -130,23 +135,39 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   // tiles of the same query heads a few tiles apart and share every HBM fetch through L2),
   // or one tile for small causal problems, where longest-tile-first over all heads matters
   // more.
+  // Packed sequences: kv heads fastest, then the tiles of all sequences, longest walk first.
   int w = blockIdx.x;
-  const int qs = w % p.q_split;
-  w /= p.q_split;
-  const int kv_lo = w % p.chunk;
-  w /= p.chunk;
-  const int g = w % p.Hkv;
-  w /= p.Hkv;
-  const int b = w % p.B;
-  const int kvblk = (w / p.B) * p.chunk + kv_lo;
+  int qs = 0, g, b, kvblk, sg = 0;
+  if constexpr (kVar) {
+    g = w % p.Hkv;
+    b = 0;
+    const int left = var.decode(w / p.Hkv, sg);   // tiles behind this one in its sequence
+    kvblk = var.seq(sg).nblk - 1 - left;
+  } else {
+    qs = w % p.q_split;
+    w /= p.q_split;
+    const int kv_lo = w % p.chunk;
+    w /= p.chunk;
+    g = w % p.Hkv;
+    w /= p.Hkv;
+    b = w % p.B;
+    kvblk = (w / p.B) * p.chunk + kv_lo;
+  }
+  const int Sq = kVar ? var.seq(sg).sq : p.Sq;
+  const int Sk = kVar ? var.seq(sg).sk : p.Sk;
+  const int causal_off = kVar ? var.seq(sg).off : p.causal_off;
+  const int q_row0 = kVar ? var.seq(sg).q0 : 0;   // first row of the sequence in the packed tensors
+  const int k_row0 = kVar ? var.seq(sg).k0 : 0;
+  const CUtensorMap* const q_map = kVar ? var.map(sg, 0) : &tm_q;
+  const CUtensorMap* const do_map = kVar ? var.map(sg, 1) : &tm_do;
   const int kv0 = kvblk * kTileKV;
   const int G = p.Hq / p.Hkv;
 
   // Query tiles that can see this K/V tile.
-  int i_end = (p.Sq + kTileQ - 1) / kTileQ;
+  int i_end = (Sq + kTileQ - 1) / kTileQ;
   int i_start = 0;
   if (p.causal) {
-    const long long first_q = (long long)kv0 - p.causal_off;  // smallest query index seeing kv0
+    const long long first_q = (long long)kv0 - causal_off;  // smallest query index seeing kv0
     if (first_q > 0) i_start = (int)min((long long)i_end, first_q / kTileQ);
   }
   if (p.q_split > 1) {  // this CTA's slice of the visible query tiles
@@ -188,14 +209,14 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA
     if (lane == 0 && n_it > 0) {
-      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(q_map);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
-      tma_prefetch_desc(&tm_do);
+      tma_prefetch_desc(do_map);
       mbar_arrive_expect_tx(kv_full, 2 * L::kTile);
       for (int s = 0; s < D / 64; ++s) {
-        tma_load_4d(smem + L::kKOff + s * L::kSlab, &tm_k, kv_full, s * 64, kv0, g, b);
-        tma_load_4d(smem + L::kVOff + s * L::kSlab, &tm_v, kv_full, s * 64, kv0, g, b);
+        tma_load_4d(smem + L::kKOff + s * L::kSlab, &tm_k, kv_full, s * 64, k_row0 + kv0, g, b);
+        tma_load_4d(smem + L::kVOff + s * L::kSlab, &tm_v, kv_full, s * 64, k_row0 + kv0, g, b);
       }
       for (int n = 0; n < 2 * n_it; ++n) {       // n even: Q tile, n odd: dO tile
         const int slot = n % kRing;
@@ -205,7 +226,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
         const int hq = g * G + it / n_q;
         const int q0 = (i_start + it % n_q) * kTileQ;
         uint8_t* st = smem + L::kRingOff + slot * L::kTile;
-        const CUtensorMap* tm = (n & 1) ? &tm_do : &tm_q;
+        const CUtensorMap* tm = (n & 1) ? do_map : q_map;
         mbar_arrive_expect_tx(&tile_full[slot], L::kTile);
         for (int s = 0; s < D / 64; ++s)
           tma_load_4d(st + s * L::kSlab, tm, &tile_full[slot], s * 64, q0, hq, b);
@@ -309,7 +330,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
     const uint32_t t_dp = tmem_base + lane_field + kColDP + c_base;    // dP^T, then dS^T in [0,16)
     const uint32_t t_dv = tmem_base + lane_field + kColDV;
     const uint32_t t_dk = tmem_base + lane_field + kColDK;
-    const bool key_ok = kidx < p.Sk;
+    const bool key_ok = kidx < Sk;
     bool ok = true;
 
     // Row statistics of a query tile, fetched by the first 256 compute threads and stored
@@ -322,9 +343,9 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
     auto fetch_rowstat = [&](int it) -> float {
       const int hq = g * G + it / n_q;
       const int qi = (i_start + it % n_q) * kTileQ + (stat_tid & 127);
-      const size_t idx = (size_t)b * p.lse_sb + (size_t)hq * p.lse_sh + qi;
-      if (stat_tid < 128) return qi < p.Sq ? -p.lse[idx] * kLog2e : -INFINITY;
-      return qi < p.Sq ? -p.delta[idx] : 0.f;
+      const size_t idx = (size_t)b * p.lse_sb + (size_t)hq * p.lse_sh + q_row0 + qi;
+      if (stat_tid < 128) return qi < Sq ? -p.lse[idx] * kLog2e : -INFINITY;
+      return qi < Sq ? -p.delta[idx] : 0.f;
     };
     if (n_it > 0 && stat_tid < 256) {
       row_buf[(0 * 2 + (stat_tid >> 7)) * kTileQ + (stat_tid & 127)] = fetch_rowstat(0);
@@ -346,8 +367,8 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int q0 = (i_start + it % n_q) * kTileQ;
       // warp-uniform: does any row of this tile mask a column of this group?
       // (key kidx is visible to query column c iff c >= kidx - off - q0 - c_base)
-      const bool need_mask = !(kv0 + kTileKV <= p.Sk) ||
-                             (p.causal && (long long)kv0 + kTileKV - 1 - p.causal_off > (long long)q0 + c_base);
+      const bool need_mask = !(kv0 + kTileKV <= Sk) ||
+                             (p.causal && (long long)kv0 + kTileKV - 1 - causal_off > (long long)q0 + c_base);
 
       ok = warp_wait(s_full, it & 1, wc, 9, it);
       if (!ok) break;
@@ -377,9 +398,9 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
           for (int rr = 0; rr < 2; ++rr) {
             const int krow = kv0 + quad * 32 + hh * 16 + rr * 8 + g8;
             long long cm = 0;
-            if (p.causal) cm = (long long)krow - p.causal_off - q0 - c_base;
+            if (p.causal) cm = (long long)krow - causal_off - q0 - c_base;
             int c_min = (int)max(0ll, min(cm, 32ll));
-            if (krow >= p.Sk) c_min = 32;
+            if (krow >= Sk) c_min = 32;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float* e = pr + hh * 16 + 4 * i + 2 * rr;
@@ -504,7 +525,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
       }
     } else if (ok) {
-      const size_t row_off = (size_t)b * p.dkv_sb + (size_t)kidx * p.dkv_ss + (size_t)g * p.dkv_sh +
+      const size_t row_off = (size_t)b * p.dkv_sb + (size_t)(k_row0 + kidx) * p.dkv_ss + (size_t)g * p.dkv_sh +
                              grp * kCols;
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
@@ -570,8 +591,8 @@ int choose_q_split(const spa_bwd_args* a, long long base_grid) {
   return best;
 }
 
-template <int D, typename T>
-int launch_dkv_typed(const spa_bwd_args* a, int is_bf16) {
+template <int D, typename T, bool kVar>
+int launch_dkv_typed(const spa_bwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq) {
   using L = DkvSmem<D>;
   CUtensorMap tq, tk, tv, tdo, tdk, tdv;
   if (encode_rows_map(&tq, a->q, is_bf16, D, a->Sq, a->Hq, a->B, a->q_ss, a->q_sh, a->q_sb, kTileQ))
@@ -603,10 +624,22 @@ int launch_dkv_typed(const spa_bwd_args* a, int is_bf16) {
   p.status = device_status_word();
   if (!p.status) return SPA_ECUDA;
   const int smem_bytes = L::kTotal + 1024;
-  auto kern = attn_bwd_dkv_sm100_kernel<D, T>;
+  auto kern = attn_bwd_dkv_sm100_kernel<D, T, kVar>;
   int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd dkv sm100");
   if (rc) return rc;
-  const long long grid = (long long)p.n_kvblk * a->B * a->Hkv * p.q_split;
+  long long grid = (long long)p.n_kvblk * a->B * a->Hkv * p.q_split;
+  VarTable<kVar, 2> var;
+  if constexpr (kVar) {
+    grid = fill_var_table(&var, seqs, n_seq, kTileKV, /*by_key=*/true) * a->Hkv;
+    for (int i = 0; i < n_seq; ++i) {
+      const VarSeq& q = var.s[i];
+      if (encode_rows_map(&var.tm[i][0], row_ptr(a->q, q.q0, a->q_ss), is_bf16, D, q.sq, a->Hq, 1, a->q_ss,
+                          a->q_sh, a->q_sb, kTileQ) ||
+          encode_rows_map(&var.tm[i][1], row_ptr(a->dout, q.q0, a->do_ss), is_bf16, D, q.sq, a->Hq, 1,
+                          a->do_ss, a->do_sh, a->do_sb, kTileQ))
+        return SPA_ECUDA;
+    }
+  }
   if (grid <= 0 || grid > 0x7fffffffll) {
     set_error("bwd dkv grid out of range");
     return SPA_EINVAL;
@@ -620,7 +653,7 @@ int launch_dkv_typed(const spa_bwd_args* a, int is_bf16) {
       return SPA_ECUDA;
     }
   }
-  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, tdo, tdk, tdv, p);
+  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, tdo, tdk, tdv, p, var);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("bwd dkv sm100 launch: %s", cudaGetErrorString(e));
@@ -629,9 +662,8 @@ int launch_dkv_typed(const spa_bwd_args* a, int is_bf16) {
   return SPA_OK;
 }
 
-}  // namespace
-
-int launch_bwd_dkv_sm100(const spa_bwd_args* a) {
+template <bool kVar>
+int launch_dkv_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
   const bool bf = a->dtype == SPA_DTYPE_BF16;
   if (!a->dkv_fp32 &&
       (((uintptr_t)a->dk & 15) || ((uintptr_t)a->dv & 15) || ((a->dkv_ss * 2) & 15) ||
@@ -640,12 +672,22 @@ int launch_bwd_dkv_sm100(const spa_bwd_args* a) {
     return SPA_EINVAL;
   }
   if (a->D == 128) {
-    return bf ? launch_dkv_typed<128, __nv_bfloat16>(a, 1) : launch_dkv_typed<128, __half>(a, 0);
+    return bf ? launch_dkv_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
+              : launch_dkv_typed<128, __half, kVar>(a, 0, seqs, n_seq);
   } else if (a->D == 64) {
-    return bf ? launch_dkv_typed<64, __nv_bfloat16>(a, 1) : launch_dkv_typed<64, __half>(a, 0);
+    return bf ? launch_dkv_typed<64, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
+              : launch_dkv_typed<64, __half, kVar>(a, 0, seqs, n_seq);
   }
   set_error("tensor-core backward supports head_dim 64 and 128, got %d", a->D);
   return SPA_EUNSUPPORTED;
+}
+
+}  // namespace
+
+int launch_bwd_dkv_sm100(const spa_bwd_args* a) { return launch_dkv_any<false>(a, nullptr, 0); }
+
+int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
+  return launch_dkv_any<true>(a, seqs, n_seq);
 }
 
 }  // namespace spa

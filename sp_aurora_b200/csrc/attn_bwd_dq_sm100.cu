@@ -34,6 +34,7 @@
 
 #include "spa_internal.h"
 #include "tc05.cuh"
+#include "varlen.cuh"
 
 namespace spa {
 namespace {
@@ -90,11 +91,14 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int D, typename T>
+// kVar: one launch over the sequences of a packed batch (B = 1); K and V are then read through
+// the maps of the sequence's table entry, dO through tm_do over the whole packed tensor.
+template <int D, typename T, bool kVar>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v,
-                         const __grid_constant__ CUtensorMap tm_do, const DqParams p) {
+                         const __grid_constant__ CUtensorMap tm_do, const DqParams p,
+                         const __grid_constant__ VarTable<kVar, 2> var) {
   using L = DqSmem<D>;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   extern __shared__ uint8_t smem_raw[];
@@ -117,20 +121,34 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
 
   // Work decode: query tiles of one chunk fastest (longest first under a causal mask),
   // then heads, batch, chunks; the CTAs resident together stream the K/V of one kv head.
+  // Packed sequences: heads fastest, then the tiles of all sequences, longest walk first.
   int w = blockIdx.x;
-  const int q_lo = w % p.chunk;
-  w /= p.chunk;
-  const int h = w % p.Hq;
-  w /= p.Hq;
-  const int b = w % p.B;
-  const int qblk = p.n_qblk - 1 - ((w / p.B) * p.chunk + q_lo);
+  int h, b, qblk, sg = 0;
+  if constexpr (kVar) {
+    h = w % p.Hq;
+    b = 0;
+    qblk = var.decode(w / p.Hq, sg);
+  } else {
+    const int q_lo = w % p.chunk;
+    w /= p.chunk;
+    h = w % p.Hq;
+    w /= p.Hq;
+    b = w % p.B;
+    qblk = p.n_qblk - 1 - ((w / p.B) * p.chunk + q_lo);
+  }
+  const int Sq = kVar ? var.seq(sg).sq : p.Sq;
+  const int Sk = kVar ? var.seq(sg).sk : p.Sk;
+  const int causal_off = kVar ? var.seq(sg).off : p.causal_off;
+  const int q_row0 = kVar ? var.seq(sg).q0 : 0;   // first row of the sequence in the packed tensors
+  const CUtensorMap* const k_map = kVar ? var.map(sg, 0) : &tm_k;
+  const CUtensorMap* const v_map = kVar ? var.map(sg, 1) : &tm_v;
   const int hk = h / (p.Hq / p.Hkv);
   const int q0 = qblk * kTileM;
 
   // K/V tiles this query tile can see.
-  int n_kv = (p.Sk + kTileN - 1) / kTileN;
+  int n_kv = (Sk + kTileN - 1) / kTileN;
   if (p.causal) {
-    const long long last_key = (long long)min(q0 + kTileM, p.Sq) - 1 + p.causal_off;  // inclusive
+    const long long last_key = (long long)min(q0 + kTileM, Sq) - 1 + causal_off;  // inclusive
     const int nc = last_key < 0 ? 0 : (int)(last_key / kTileN) + 1;
     n_kv = min(n_kv, nc);
   }
@@ -163,12 +181,12 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
   if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA
     if (lane == 0 && n_kv > 0) {
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
+      tma_prefetch_desc(k_map);
+      tma_prefetch_desc(v_map);
       tma_prefetch_desc(&tm_do);
       mbar_arrive_expect_tx(do_full, L::kTile);
       for (int s = 0; s < D / 64; ++s)
-        tma_load_4d(smem + L::kDoOff + s * L::kSlab, &tm_do, do_full, s * 64, q0, h, b);
+        tma_load_4d(smem + L::kDoOff + s * L::kSlab, &tm_do, do_full, s * 64, q_row0 + q0, h, b);
       for (int j = 0; j < n_kv; ++j) {
         const int slot = j % kStages;
         const uint32_t ph = (j / kStages) & 1;
@@ -176,8 +194,8 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
         uint8_t* st = smem + L::kKVOff + slot * L::kStageBytes;
         mbar_arrive_expect_tx(&kv_full[slot], L::kStageBytes);
         for (int s = 0; s < D / 64; ++s) {
-          tma_load_4d(st + s * L::kSlab, &tm_k, &kv_full[slot], s * 64, j * kTileN, hk, b);
-          tma_load_4d(st + L::kTile + s * L::kSlab, &tm_v, &kv_full[slot], s * 64, j * kTileN, hk, b);
+          tma_load_4d(st + s * L::kSlab, k_map, &kv_full[slot], s * 64, j * kTileN, hk, b);
+          tma_load_4d(st + L::kTile + s * L::kSlab, v_map, &kv_full[slot], s * 64, j * kTileN, hk, b);
         }
       }
     }
@@ -255,7 +273,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
     const int quad = warp & 3;
     const int r = quad * 32 + lane;            // query row in tile = TMEM lane
     const int qrow = q0 + r;
-    const bool row_ok = qrow < p.Sq;
+    const bool row_ok = qrow < Sq;
     const int c_base = grp * 32;
     constexpr int kOutCols = D / 4;            // dQ columns (and Q elements) per group
     const uint32_t lane_field = static_cast<uint32_t>(quad * 32) << 16;
@@ -272,7 +290,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
       uint32_t qw[kWords];
       if (row_ok) {
         const uint4* src = reinterpret_cast<const uint4*>(
-            reinterpret_cast<const T*>(p.q) + (size_t)b * p.q_sb + (size_t)qrow * p.q_ss +
+            reinterpret_cast<const T*>(p.q) + (size_t)b * p.q_sb + (size_t)(q_row0 + qrow) * p.q_ss +
             (size_t)h * p.q_sh + grp * (D / 4));
 #pragma unroll
         for (int i = 0; i < kWords / 4; ++i) {
@@ -290,7 +308,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
     }
     // Row statistics, negated for the packed multiply-adds: -inf in place of -lse makes
     // out-of-range rows give P = 0.
-    const size_t sidx = (size_t)b * p.lse_sb + (size_t)h * p.lse_sh + (row_ok ? qrow : 0);
+    const size_t sidx = (size_t)b * p.lse_sb + (size_t)h * p.lse_sh + (row_ok ? q_row0 + qrow : 0);
     const float nlse2 = row_ok ? -p.lse[sidx] * kLog2e : -INFINITY;
     const float ndlt = row_ok ? -p.delta[sidx] : 0.f;
 
@@ -311,8 +329,8 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
 
       const int k0 = j * kTileN;
       const bool need_mask =
-          (k0 + kTileN > p.Sk) ||
-          (p.causal && ((long long)k0 + kTileN - 1 > (long long)q0 + p.causal_off));
+          (k0 + kTileN > Sk) ||
+          (p.causal && ((long long)k0 + kTileN - 1 > (long long)q0 + causal_off));
       if (!need_mask) {                            // tiles below the diagonal: no selects
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
@@ -322,8 +340,8 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
           pr[c + 1] = fast_exp2(x1);
         }
       } else {
-        long long lim = p.Sk - 1;
-        if (p.causal) lim = min(lim, (long long)qrow + p.causal_off);
+        long long lim = Sk - 1;
+        if (p.causal) lim = min(lim, (long long)qrow + causal_off);
         const int limit = (int)max(0ll, min(lim - k0 - c_base + 1, 32ll));   // first masked column
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
@@ -364,7 +382,7 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
       const size_t acc_off = (((size_t)b * p.Sq + qrow) * p.Hq + h) * D + grp * kOutCols;
       const float* acc_in = (!p.dq_overwrite && p.dq_acc) ? p.dq_acc + acc_off : nullptr;
       float* acc_out = p.dq_acc ? p.dq_acc + acc_off : nullptr;
-      T* out_row = p.dq ? reinterpret_cast<T*>(p.dq) + (size_t)b * p.dq_sb + (size_t)qrow * p.dq_ss +
+      T* out_row = p.dq ? reinterpret_cast<T*>(p.dq) + (size_t)b * p.dq_sb + (size_t)(q_row0 + qrow) * p.dq_ss +
                               (size_t)h * p.dq_sh + grp * kOutCols
                         : nullptr;
       const bool skip = (n_kv == 0) && !p.dq_overwrite && !p.dq;   // the accumulator already holds the total
@@ -419,8 +437,8 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
   }
 }
 
-template <int D, typename T>
-int launch_dq_typed(const spa_bwd_args* a, int is_bf16) {
+template <int D, typename T, bool kVar>
+int launch_dq_typed(const spa_bwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq) {
   using L = DqSmem<D>;
   CUtensorMap tk, tv, tdo;
   if (encode_rows_map(&tdo, a->dout, is_bf16, D, a->Sq, a->Hq, a->B, a->do_ss, a->do_sh, a->do_sb,
@@ -443,15 +461,27 @@ int launch_dq_typed(const spa_bwd_args* a, int is_bf16) {
   p.status = device_status_word();
   if (!p.status) return SPA_ECUDA;
   const int smem_bytes = L::kTotal + 1024;
-  auto kern = attn_bwd_dq_sm100_kernel<D, T>;
+  auto kern = attn_bwd_dq_sm100_kernel<D, T, kVar>;
   int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "bwd dq sm100");
   if (rc) return rc;
-  const long long grid = (long long)p.n_qblk * a->B * a->Hq;
+  long long grid = (long long)p.n_qblk * a->B * a->Hq;
+  VarTable<kVar, 2> var;
+  if constexpr (kVar) {
+    grid = fill_var_table(&var, seqs, n_seq, kTileM, /*by_key=*/false) * a->Hq;
+    for (int i = 0; i < n_seq; ++i) {
+      const VarSeq& q = var.s[i];
+      if (encode_rows_map(&var.tm[i][0], row_ptr(a->k, q.k0, a->k_ss), is_bf16, D, q.sk, a->Hkv, 1, a->k_ss,
+                          a->k_sh, a->k_sb, kTileN) ||
+          encode_rows_map(&var.tm[i][1], row_ptr(a->v, q.k0, a->v_ss), is_bf16, D, q.sk, a->Hkv, 1, a->v_ss,
+                          a->v_sh, a->v_sb, kTileN))
+        return SPA_ECUDA;
+    }
+  }
   if (grid <= 0 || grid > 0x7fffffffll) {
     set_error("bwd dq grid out of range");
     return SPA_EINVAL;
   }
-  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tk, tv, tdo, p);
+  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tk, tv, tdo, p, var);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("bwd dq sm100 launch: %s", cudaGetErrorString(e));
@@ -460,21 +490,30 @@ int launch_dq_typed(const spa_bwd_args* a, int is_bf16) {
   return SPA_OK;
 }
 
-}  // namespace
-
-int launch_bwd_dq_sm100(const spa_bwd_args* a) {
+template <bool kVar>
+int launch_dq_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
   const bool bf = a->dtype == SPA_DTYPE_BF16;
   if (((uintptr_t)a->q & 15) || ((a->q_ss * 2) & 15) || ((a->q_sh * 2) & 15) || ((a->q_sb * 2) & 15)) {
     set_error("q base and strides must be 16-byte aligned");
     return SPA_EINVAL;
   }
   if (a->D == 128) {
-    return bf ? launch_dq_typed<128, __nv_bfloat16>(a, 1) : launch_dq_typed<128, __half>(a, 0);
+    return bf ? launch_dq_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
+              : launch_dq_typed<128, __half, kVar>(a, 0, seqs, n_seq);
   } else if (a->D == 64) {
-    return bf ? launch_dq_typed<64, __nv_bfloat16>(a, 1) : launch_dq_typed<64, __half>(a, 0);
+    return bf ? launch_dq_typed<64, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
+              : launch_dq_typed<64, __half, kVar>(a, 0, seqs, n_seq);
   }
   set_error("tensor-core backward supports head_dim 64 and 128, got %d", a->D);
   return SPA_EUNSUPPORTED;
+}
+
+}  // namespace
+
+int launch_bwd_dq_sm100(const spa_bwd_args* a) { return launch_dq_any<false>(a, nullptr, 0); }
+
+int launch_bwd_dq_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
+  return launch_dq_any<true>(a, seqs, n_seq);
 }
 
 }  // namespace spa

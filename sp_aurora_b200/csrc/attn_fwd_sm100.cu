@@ -25,6 +25,7 @@
 
 #include "spa_internal.h"
 #include "tc05.cuh"
+#include "varlen.cuh"
 
 namespace spa {
 
@@ -76,11 +77,14 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int D, typename T>
+// kVar: one launch over the sequences of a packed batch (B = 1). tm_q and tm_k then cover the
+// whole packed tensors, the V map comes from the sequence's table entry (see varlen.cuh).
+template <int D, typename T, bool kVar>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
                       const __grid_constant__ CUtensorMap tm_k,
-                      const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
+                      const __grid_constant__ CUtensorMap tm_v, const FwdParams p,
+                      const __grid_constant__ VarTable<kVar, 1> var) {
   using L = FwdSmem<D>;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   extern __shared__ uint8_t smem_raw[];
@@ -104,14 +108,28 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   // then heads, batch, chunks. The host picks the chunk: all query blocks (CTAs resident
   // together then stream the K/V of one kv head, which stays in L2: S=131072 causal
   // 993 -> 1036 TFLOP/s), or one block for small causal problems, where
-  // longest-block-first over all heads matters more.
+  // longest-block-first over all heads matters more. Packed sequences: heads fastest, then
+  // the blocks of all sequences by falling distance from the start of their sequence.
   int w = blockIdx.x;
-  const int q_lo = w % p.chunk;
-  w /= p.chunk;
-  const int h = w % p.Hq;
-  w /= p.Hq;
-  const int b = w % p.B;
-  const int qblk = p.n_qblk - 1 - ((w / p.B) * p.chunk + q_lo);
+  int h, b, qblk, sg = 0;
+  if constexpr (kVar) {
+    h = w % p.Hq;
+    b = 0;
+    qblk = var.decode(w / p.Hq, sg);
+  } else {
+    const int q_lo = w % p.chunk;
+    w /= p.chunk;
+    h = w % p.Hq;
+    w /= p.Hq;
+    b = w % p.B;
+    qblk = p.n_qblk - 1 - ((w / p.B) * p.chunk + q_lo);
+  }
+  const int Sq = kVar ? var.seq(sg).sq : p.Sq;
+  const int Sk = kVar ? var.seq(sg).sk : p.Sk;
+  const int causal_off = kVar ? var.seq(sg).off : p.causal_off;
+  const int q_row0 = kVar ? var.seq(sg).q0 : 0;   // first row of the sequence in the packed tensors
+  const int k_row0 = kVar ? var.seq(sg).k0 : 0;
+  const CUtensorMap* const v_map = kVar ? var.map(sg, 0) : &tm_v;
   const int hk = h / (p.Hq / p.Hkv);
   const int q0 = qblk * 2 * kTileM;
 
@@ -121,11 +139,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   for (int t = 0; t < 2; ++t) {
     const int r0 = q0 + t * kTileM;
     int n = 0;
-    if (r0 < p.Sq) {
-      n = (p.Sk + kTileN - 1) / kTileN;
+    if (r0 < Sq) {
+      n = (Sk + kTileN - 1) / kTileN;
       if (p.causal) {
-        const int last_row = min(r0 + kTileM, p.Sq) - 1;
-        const long long last_key = (long long)last_row + p.causal_off;  // inclusive
+        const int last_row = min(r0 + kTileM, Sq) - 1;
+        const long long last_key = (long long)last_row + causal_off;  // inclusive
         const int nc = last_key < 0 ? 0 : (int)(last_key / kTileN) + 1;
         n = min(n, nc);
       }
@@ -164,24 +182,25 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
     if (lane == 0 && nmax > 0) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      const int q_tiles = (n_t[1] > 0 || q0 + kTileM < p.Sq) ? 2 : 1;
+      tma_prefetch_desc(v_map);
+      const int q_tiles = (n_t[1] > 0 || q0 + kTileM < Sq) ? 2 : 1;
       mbar_arrive_expect_tx(q_full, q_tiles * L::kTileBytes);
       for (int t = 0; t < q_tiles; ++t)
         for (int s = 0; s < D / 64; ++s)
           tma_load_4d(smem + L::kQOff + t * L::kTileBytes + s * L::kSlabBytes, &tm_q, q_full,
-                      s * 64, q0 + t * kTileM, h, b);
+                      s * 64, q_row0 + q0 + t * kTileM, h, b);
       const int nfill = 2 * nmax;
       for (int n = 0; n < nfill; ++n) {
         const int slot = n % L::kStages;
         const uint32_t ph = (n / L::kStages) & 1;
         if (!mbar_wait(&kv_empty[slot], ph ^ 1, wc, 0, n)) break;
         mbar_arrive_expect_tx(&kv_full[slot], L::kTileBytes);
-        const CUtensorMap* tm = (n & 1) ? &tm_v : &tm_k;
+        const CUtensorMap* tm = (n & 1) ? v_map : &tm_k;
         const int j = n >> 1;
+        const int row = j * kTileN + ((n & 1) ? 0 : k_row0);
         for (int s = 0; s < D / 64; ++s)
           tma_load_4d(smem + L::kKVOff + slot * L::kTileBytes + s * L::kSlabBytes, tm,
-                      &kv_full[slot], s * 64, j * kTileN, hk, b);
+                      &kv_full[slot], s * 64, row, hk, b);
       }
     }
   } else if (warp == 9) {
@@ -288,12 +307,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       float* s = reinterpret_cast<float*>(sr);
 
       const int k0 = j * kTileN;
-      const bool need_mask = (k0 + kTileN > p.Sk) ||
+      const bool need_mask = (k0 + kTileN > Sk) ||
                              (p.causal && ((long long)k0 + kTileN - 1 >
-                                           (long long)tile_row_min + p.causal_off));
+                                           (long long)tile_row_min + causal_off));
       if (need_mask) {
-        long long lim = p.Sk - 1;
-        if (p.causal) lim = min(lim, (long long)qrow + p.causal_off);
+        long long lim = Sk - 1;
+        if (p.causal) lim = min(lim, (long long)qrow + causal_off);
         const int limit = (int)max(-1ll, min(lim - k0, 127ll));  // last visible column
 #pragma unroll
         for (int c = 0; c < 128; ++c)
@@ -358,11 +377,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       tc_fence_after();
     }
     if (ok) {
-      const bool row_ok = qrow < p.Sq;
+      const bool row_ok = qrow < Sq;
       const bool have = (nt > 0) && (l > 0.f);
       const float inv_l = have ? 1.f / l : 0.f;
       const float lse_blk = have ? (m_used + log2f(l)) * kLn2 : ninf;
-      const size_t lse_idx = (size_t)b * p.lse_sb + (size_t)h * p.lse_sh + qrow;
+      const size_t lse_idx = (size_t)b * p.lse_sb + (size_t)h * p.lse_sh + q_row0 + qrow;
       float w_old = 0.f, w_blk = have ? 1.f : 0.f, lse_new = lse_blk;
       if (p.merge_prev && row_ok) {
         const float lse_old = p.lse[lse_idx];
@@ -385,7 +404,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       float* acc_row =
           p.out_acc ? p.out_acc + (((size_t)b * p.Sq + qrow) * p.Hq + h) * D : nullptr;
       T* out_row = p.out ? reinterpret_cast<T*>(p.out) + (size_t)b * p.o_sb +
-                               (size_t)qrow * p.o_ss + (size_t)h * p.o_sh
+                               (size_t)(q_row0 + qrow) * p.o_ss + (size_t)h * p.o_sh
                          : nullptr;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
@@ -443,8 +462,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
 }
 
-template <int D, typename T>
-int launch_fwd_typed(const spa_fwd_args* a, int is_bf16) {
+template <int D, typename T, bool kVar>
+int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq) {
   using L = FwdSmem<D>;
   CUtensorMap tq, tk, tv;
   if (encode_rows_map(&tq, a->q, is_bf16, D, a->Sq, a->Hq, a->B, a->q_ss, a->q_sh, a->q_sb, kTileM))
@@ -464,15 +483,25 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16) {
   p.status = device_status_word();
   if (!p.status) return SPA_ECUDA;
   const int smem_bytes = L::kTotal + 1024;
-  auto kern = attn_fwd_sm100_kernel<D, T>;
+  auto kern = attn_fwd_sm100_kernel<D, T, kVar>;
   int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "fwd sm100");
   if (rc) return rc;
-  const long long grid = (long long)p.n_qblk * a->B * a->Hq;
+  long long grid = (long long)p.n_qblk * a->B * a->Hq;
+  VarTable<kVar, 1> var;
+  if constexpr (kVar) {
+    grid = fill_var_table(&var, seqs, n_seq, 2 * kTileM, /*by_key=*/false) * a->Hq;
+    for (int i = 0; i < n_seq; ++i) {
+      const VarSeq& q = var.s[i];
+      if (encode_rows_map(&var.tm[i][0], row_ptr(a->v, q.k0, a->v_ss), is_bf16, D, q.sk, a->Hkv, 1, a->v_ss,
+                          a->v_sh, a->v_sb, kTileN))
+        return SPA_ECUDA;
+    }
+  }
   if (grid <= 0 || grid > 0x7fffffffll) {
     set_error("fwd grid out of range");
     return SPA_EINVAL;
   }
-  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, p);
+  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, p, var);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("fwd sm100 launch: %s", cudaGetErrorString(e));
@@ -481,17 +510,26 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16) {
   return SPA_OK;
 }
 
-}  // namespace
-
-int launch_fwd_sm100(const spa_fwd_args* a) {
+template <bool kVar>
+int launch_fwd_any(const spa_fwd_args* a, const spa_seq* seqs, int n_seq) {
   const bool bf = a->dtype == SPA_DTYPE_BF16;
   if (a->D == 128) {
-    return bf ? launch_fwd_typed<128, __nv_bfloat16>(a, 1) : launch_fwd_typed<128, __half>(a, 0);
+    return bf ? launch_fwd_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
+              : launch_fwd_typed<128, __half, kVar>(a, 0, seqs, n_seq);
   } else if (a->D == 64) {
-    return bf ? launch_fwd_typed<64, __nv_bfloat16>(a, 1) : launch_fwd_typed<64, __half>(a, 0);
+    return bf ? launch_fwd_typed<64, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
+              : launch_fwd_typed<64, __half, kVar>(a, 0, seqs, n_seq);
   }
   set_error("tensor-core forward supports head_dim 64 and 128, got %d", a->D);
   return SPA_EUNSUPPORTED;
+}
+
+}  // namespace
+
+int launch_fwd_sm100(const spa_fwd_args* a) { return launch_fwd_any<false>(a, nullptr, 0); }
+
+int launch_fwd_sm100_var(const spa_fwd_args* a, const spa_seq* seqs, int n_seq) {
+  return launch_fwd_any<true>(a, seqs, n_seq);
 }
 
 }  // namespace spa

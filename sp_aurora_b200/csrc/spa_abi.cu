@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "spa_internal.h"
+#include "varlen.cuh"
 
 namespace spa {
 
@@ -739,26 +740,27 @@ static bool misaligned(const void* p, int64_t sb, int64_t ss, int64_t sh, int el
 }
 static int elt_size(int dtype) { return dtype == SPA_DTYPE_F32 ? 4 : 2; }
 
-int spa_attn_fwd(const spa_fwd_args* args) {
+// Fills in the defaults of *args and checks them; the normalised arguments go to *n.
+static int prepare_fwd(const spa_fwd_args* args, spa_fwd_args* n, const char* what) {
   if (!args || !args->q || !args->k || !args->v || !args->lse) {
-    set_error("spa_attn_fwd: null pointer argument");
+    set_error("%s: null pointer argument", what);
     return SPA_EINVAL;
   }
-  spa_fwd_args n = *args;
-  const spa_fwd_args* a = &n;
+  *n = *args;
+  const spa_fwd_args* a = n;
   int rc = validate_common(a->B, a->Sq, a->Sk, a->Hq, a->Hkv, a->D, a->dtype, a->scale);
   if (rc) return rc;
   if (!a->out && !a->out_acc) {
-    set_error("spa_attn_fwd: at least one of out / out_acc is required");
+    set_error("%s: at least one of out / out_acc is required", what);
     return SPA_EINVAL;
   }
   if (a->merge_prev && !a->out_acc) {
-    set_error("spa_attn_fwd: merge_prev needs out_acc");
+    set_error("%s: merge_prev needs out_acc", what);
     return SPA_EINVAL;
   }
-  if (n.lse_sb == 0 && n.lse_sh == 0) {
-    n.lse_sh = a->Sq;
-    n.lse_sb = (int64_t)a->Hq * a->Sq;
+  if (n->lse_sb == 0 && n->lse_sh == 0) {
+    n->lse_sh = a->Sq;
+    n->lse_sb = (int64_t)a->Hq * a->Sq;
   }
   // Rows are read and written as 16-byte vectors by every kernel.
   const int es = elt_size(a->dtype);
@@ -767,12 +769,78 @@ int spa_attn_fwd(const spa_fwd_args* args) {
       misaligned(a->v, a->v_sb, a->v_ss, a->v_sh, es, 16) ||
       (a->out && misaligned(a->out, a->o_sb, a->o_ss, a->o_sh, es, 16)) ||
       (a->out_acc && ((uintptr_t)a->out_acc & 15))) {
-    set_error("spa_attn_fwd: tensor bases and strides must be multiples of 16 bytes");
+    set_error("%s: tensor bases and strides must be multiples of 16 bytes", what);
     return SPA_EINVAL;
   }
-  const bool tensor_core = a->dtype != SPA_DTYPE_F32 && a->D != 32 && !force_simt();
-  rc = tensor_core ? launch_fwd_sm100(a) : launch_fwd_simt(a);
+  return SPA_OK;
+}
+
+static bool on_tensor_cores(int dtype, int D) { return dtype != SPA_DTYPE_F32 && D != 32 && !force_simt(); }
+
+int spa_attn_fwd(const spa_fwd_args* args) {
+  spa_fwd_args n;
+  int rc = prepare_fwd(args, &n, "spa_attn_fwd");
+  if (rc) return rc;
+  rc = on_tensor_cores(n.dtype, n.D) ? launch_fwd_sm100(&n) : launch_fwd_simt(&n);
   if (rc == SPA_OK) note_launch(1);
+  return rc;
+}
+
+static int validate_seqs(const spa_seq* seqs, int n, int B, int Sq, int Sk, const char* what) {
+  if (!seqs || n <= 0 || B != 1) {
+    set_error("%s: needs B = 1 and at least one sequence", what);
+    return SPA_EINVAL;
+  }
+  long long q_end = 0, k_end = 0;
+  for (int i = 0; i < n; ++i) {
+    const spa_seq& q = seqs[i];
+    if (q.sq <= 0 || q.sk <= 0 || q.q0 < q_end || q.k0 < k_end || (long long)q.q0 + q.sq > Sq ||
+        (long long)q.k0 + q.sk > Sk) {
+      set_error("%s: sequence %d (queries %d+%d of %d, keys %d+%d of %d) is empty, out of order or out of range",
+                what, i, q.q0, q.sq, Sq, q.k0, q.sk, Sk);
+      return SPA_EINVAL;
+    }
+    q_end = (long long)q.q0 + q.sq;
+    k_end = (long long)q.k0 + q.sk;
+  }
+  return SPA_OK;
+}
+
+static const void* seq_row(const void* base, int64_t row, int64_t stride, int es) {
+  return static_cast<const char*>(base) + row * stride * es;
+}
+
+int spa_attn_varlen_fwd(const spa_fwd_args* args, const spa_seq* seqs, int32_t n_seq) {
+  spa_fwd_args n;
+  int rc = prepare_fwd(args, &n, "spa_attn_varlen_fwd");
+  if (rc == SPA_OK) rc = validate_seqs(seqs, n_seq, n.B, n.Sq, n.Sk, "spa_attn_varlen_fwd");
+  if (rc) return rc;
+  if (n.merge_prev || n.out_acc) {
+    set_error("spa_attn_varlen_fwd: merge_prev / out_acc are not supported");
+    return SPA_EINVAL;
+  }
+  if (on_tensor_cores(n.dtype, n.D)) {
+    for (int i = 0; i < n_seq && rc == SPA_OK; i += kVarMaxSeqs) {
+      rc = launch_fwd_sm100_var(&n, seqs + i, std::min(kVarMaxSeqs, n_seq - i));
+      if (rc == SPA_OK) note_launch(1);
+    }
+    return rc;
+  }
+  const int es = elt_size(n.dtype);
+  for (int i = 0; i < n_seq && rc == SPA_OK; ++i) {   // CUDA cores: a launch per sequence
+    const spa_seq& q = seqs[i];
+    spa_fwd_args a = n;
+    a.q = seq_row(n.q, q.q0, n.q_ss, es);
+    a.k = seq_row(n.k, q.k0, n.k_ss, es);
+    a.v = seq_row(n.v, q.k0, n.v_ss, es);
+    a.out = const_cast<void*>(seq_row(n.out, q.q0, n.o_ss, es));
+    a.lse = n.lse + q.q0;
+    a.Sq = q.sq;
+    a.Sk = q.sk;
+    a.causal_off = q.causal_off;
+    rc = launch_fwd_simt(&a);
+    if (rc == SPA_OK) note_launch(1);
+  }
   return rc;
 }
 
@@ -836,7 +904,7 @@ static void normalise_bwd(spa_bwd_args* n) {
 
 // Both passes of the backward on the stream of `a` (already normalised and validated).
 static int run_bwd(const spa_bwd_args* a) {
-  const bool tensor_core = a->dtype != SPA_DTYPE_F32 && a->D != 32 && !force_simt();
+  const bool tensor_core = on_tensor_cores(a->dtype, a->D);
   const bool want_dq = a->passes != SPA_BWD_DKV_ONLY, want_dkv = a->passes != SPA_BWD_DQ_ONLY;
   int rc = SPA_OK;
   if (tensor_core) {
@@ -861,6 +929,53 @@ int spa_attn_bwd(const spa_bwd_args* args) {
   rc = validate_bwd(&n);
   if (rc) return rc;
   return run_bwd(&n);
+}
+
+int spa_attn_varlen_bwd(const spa_bwd_args* args, const spa_seq* seqs, int32_t n_seq) {
+  if (!args || !args->q || !args->k || !args->v || !args->dout || !args->lse || !args->delta) {
+    set_error("spa_attn_varlen_bwd: null pointer argument");
+    return SPA_EINVAL;
+  }
+  spa_bwd_args n = *args;
+  int rc = validate_common(n.B, n.Sq, n.Sk, n.Hq, n.Hkv, n.D, n.dtype, n.scale);
+  if (rc) return rc;
+  normalise_bwd(&n);
+  rc = validate_bwd(&n);
+  if (rc == SPA_OK) rc = validate_seqs(seqs, n_seq, n.B, n.Sq, n.Sk, "spa_attn_varlen_bwd");
+  if (rc) return rc;
+  if (n.passes != SPA_BWD_BOTH || n.dq_acc || !n.dq_overwrite || n.dkv_fp32 || n.dkv_accumulate) {
+    set_error("spa_attn_varlen_bwd: both passes, element-type gradients, no accumulation");
+    return SPA_EINVAL;
+  }
+  if (on_tensor_cores(n.dtype, n.D)) {
+    for (int i = 0; i < n_seq && rc == SPA_OK; i += kVarMaxSeqs) {
+      const int m = std::min(kVarMaxSeqs, n_seq - i);
+      rc = launch_bwd_dq_sm100_var(&n, seqs + i, m);
+      if (rc == SPA_OK) rc = launch_bwd_dkv_sm100_var(&n, seqs + i, m);
+      if (rc == SPA_OK) note_launch(2);
+    }
+    return rc;
+  }
+  const int es = elt_size(n.dtype);
+  for (int i = 0; i < n_seq && rc == SPA_OK; ++i) {
+    const spa_seq& q = seqs[i];
+    spa_bwd_args a = n;
+    a.q = seq_row(n.q, q.q0, n.q_ss, es);
+    a.dout = seq_row(n.dout, q.q0, n.do_ss, es);
+    a.dq = const_cast<void*>(seq_row(n.dq, q.q0, n.dq_ss, es));
+    a.k = seq_row(n.k, q.k0, n.k_ss, es);
+    a.v = seq_row(n.v, q.k0, n.v_ss, es);
+    a.dk = const_cast<void*>(seq_row(n.dk, q.k0, n.dkv_ss, es));
+    a.dv = const_cast<void*>(seq_row(n.dv, q.k0, n.dkv_ss, es));
+    a.lse = n.lse + q.q0;
+    a.delta = n.delta + q.q0;
+    a.Sq = q.sq;
+    a.Sk = q.sk;
+    a.causal_off = q.causal_off;
+    rc = launch_bwd_simt(&a);
+    if (rc == SPA_OK) note_launch(2);
+  }
+  return rc;
 }
 
 #define SPA_DISPATCH_T(dtype, ...)                                 \

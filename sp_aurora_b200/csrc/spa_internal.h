@@ -43,6 +43,10 @@ int device_sm_count();
 int launch_fwd_sm100(const spa_fwd_args* a);
 int launch_bwd_dq_sm100(const spa_bwd_args* a);       // query-stationary pass: dQ
 int launch_bwd_dkv_sm100(const spa_bwd_args* a);      // K/V-stationary pass: dK, dV
+// The same kernels over up to kVarMaxSeqs sequences of a packed batch (B = 1).
+int launch_fwd_sm100_var(const spa_fwd_args* a, const spa_seq* seqs, int n_seq);
+int launch_bwd_dq_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
+int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_fwd_simt(const spa_fwd_args* a);
 int launch_bwd_simt(const spa_bwd_args* a);
 

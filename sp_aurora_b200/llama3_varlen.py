@@ -18,6 +18,9 @@ another. Each rank attends its own query tokens to the keys of the sequences the
   backward  the same gathers; dQ straight into the result; dK/dV of a head group into an fp32
             buffer over the gathered key range, reduce-scattered to the owning ranks.
 
+On one rank there is nothing to gather: all segments and heads go through one set of kernel
+launches (spa_attn_varlen_fwd / _bwd) and dK/dV are written in the element type at once.
+
 Every query row and every key row of a head group is written by exactly one kernel call per
 rank, so nothing is accumulated on a GPU and the result does not depend on scheduling.
 """
@@ -92,6 +95,21 @@ def _segments(cu_q, cu_k) -> List[Tuple[int, int, int, int]]:
     return segs
 
 
+def _one_launch(segs, Tq: int, Tk: int) -> bool:
+    """Segments the packed kernels take as they are: rising, inside the tensors. (Tables made by
+    llama3_flash_attn_prepare_cu_seqlens always are.)"""
+    ends = [0, 0]
+    for qa, qb, ka, kb in segs:
+        if qa < ends[0] or ka < ends[1]:
+            return False
+        ends = [qb, kb]
+    return bool(segs) and ends[0] <= Tq and ends[1] <= Tk
+
+
+def _seqs(segs):
+    return [(qa, qb - qa, ka, kb - ka, (kb - ka) - (qb - qa)) for qa, qb, ka, kb in segs]
+
+
 class _Gather:
     """All-gather of one head group of K and of V: [T/W, hs, D] per rank -> [T, hs, D] each
     (rank-major along the token axis, which is the stream order)."""
@@ -137,6 +155,10 @@ def llama3_forward(group, q, k, v, segs, k_slice: slice, heads_k_stride: int, so
     g = Hq // Hkv
     out = torch.empty_like(q)
     lse = torch.empty((Hq, Tl), dtype=torch.float32, device=q.device)
+    if W == 1 and fwd_step is local_attn.attn_fwd_step and _one_launch(segs, Tl, k[k_slice].shape[0]):
+        fwd_step(q.unsqueeze(0), k[k_slice].unsqueeze(0), v[k_slice].unsqueeze(0), softmax_scale, causal,
+                 lse.unsqueeze(0), out=out.unsqueeze(0), seqs=_seqs(segs))
+        return out, lse
     gather = _Gather(group, W)
     groups = [(h0, min(h0 + heads_k_stride, Hkv)) for h0 in range(0, Hkv, heads_k_stride)]
     pending = gather.start(k, v, *groups[0])
@@ -164,6 +186,9 @@ def llama3_backward(group, dout, q, k, v, out, lse, segs, k_slice: slice, heads_
     Tl, Hq, D = q.shape
     Hkv = k.shape[1]
     g = Hq // Hkv
+    if W == 1 and bwd_step is local_attn.attn_bwd_step and _one_launch(segs, Tl, k[k_slice].shape[0]):
+        return local_attn.packed_backward(dout, q, k, v, out, lse, _seqs(segs), softmax_scale, causal,
+                                          deterministic, k_slice)
     dt = q.dtype
     acc_dt = torch.float32
     delta = delta_fn(out.unsqueeze(0), dout.unsqueeze(0))[0]          # [Hq, T/W]

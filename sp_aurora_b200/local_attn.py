@@ -84,6 +84,14 @@ def attn_flops(B, Sq, Sk, Hq, D, causal, causal_off=0) -> float:
     return 4.0 * B * Hq * D * pairs
 
 
+def _call_flops(B, Sq, Sk, Hq, D, causal, causal_off, seqs) -> float:
+    if KERNEL_TIMERS is None:
+        return 0.0
+    if seqs is None:
+        return attn_flops(B, Sq, Sk, Hq, D, causal, causal_off)
+    return sum(attn_flops(1, sq, sk, Hq, D, causal, off) for _, sq, _, sk, off in seqs)
+
+
 def check_unsupported_kwargs(dropout_p=0.0, window_size=(-1, -1), alibi_slopes=None, softcap=0.0):
     """The reference accepts and silently ignores these
     (sp_aurora/intel_flash_attn.py:25-28); here they are rejected loudly."""
@@ -145,8 +153,9 @@ def _fill_qkv(a, q, k, v):
 
 def attn_fwd_step(q, k, v, softmax_scale: float, causal: bool, lse: torch.Tensor,
                   out: Optional[torch.Tensor] = None, out_acc: Optional[torch.Tensor] = None,
-                  merge_prev: bool = False, causal_off: int = 0) -> None:
-    """One spa_attn_fwd call. `lse` fp32 [B,Hq,Sq] (rows contiguous) is written (and
+                  merge_prev: bool = False, causal_off: int = 0, seqs=None) -> None:
+    """One spa_attn_fwd call, or with `seqs` (rows (q0, sq, k0, sk, causal_off)) one
+    spa_attn_varlen_fwd call over the sequences packed in the batch-1 tensors. `lse` fp32 [B,Hq,Sq] (rows contiguous) is written (and
     read when merge_prev); `out` (q.dtype, strided) and/or `out_acc` (fp32 contiguous)
     receive the (merged) rows."""
     B, Sq, Sk, Hq, Hkv, D = check_qkv(q, k, v)
@@ -167,8 +176,11 @@ def attn_fwd_step(q, k, v, softmax_scale: float, causal: bool, lse: torch.Tensor
     a.causal, a.causal_off, a.merge_prev = int(bool(causal)), int(causal_off), int(bool(merge_prev))
     a.scale = float(softmax_scale)
     a.stream = stream_ptr(q.device)
-    with _Timed("fwd", q.device, attn_flops(B, Sq, Sk, Hq, D, causal, causal_off)):
-        check(lib.spa_attn_fwd(C.byref(a)), "spa_attn_fwd")
+    with _Timed("fwd", q.device, _call_flops(B, Sq, Sk, Hq, D, causal, causal_off, seqs)):
+        if seqs is None:
+            check(lib.spa_attn_fwd(C.byref(a)), "spa_attn_fwd")
+        else:
+            check(lib.spa_attn_varlen_fwd(C.byref(a), _lib.seq_table(seqs), len(seqs)), "spa_attn_varlen_fwd")
 
 
 def flash_attn_forward(q, k, v, softmax_scale: Optional[float] = None, causal: bool = False,
@@ -203,8 +215,9 @@ def attn_bwd_step(q, k, v, dout, lse, delta, softmax_scale: float, causal: bool,
                   dq_acc: Optional[torch.Tensor], dk: Optional[torch.Tensor],
                   dv: Optional[torch.Tensor], dkv_accumulate: bool = False, causal_off: int = 0,
                   dq: Optional[torch.Tensor] = None, dq_overwrite: bool = False,
-                  deterministic: bool = False, passes: int = _lib.SPA_BWD_BOTH) -> None:
-    """One spa_attn_bwd call (see include/spa.h). The block's dQ plus the running sum in
+                  deterministic: bool = False, passes: int = _lib.SPA_BWD_BOTH, seqs=None) -> None:
+    """One spa_attn_bwd call (see include/spa.h), or with `seqs` (as in attn_fwd_step) one
+    spa_attn_varlen_bwd call. The block's dQ plus the running sum in
     dq_acc (fp32 [B,Sq,Hq,D] contiguous; ignored on input when dq_overwrite) is written to
     dq (q.dtype, strided) and / or back to dq_acc. dk/dv [B,Sk,Hkv,D] are fp32 contiguous
     or q.dtype (strided), overwritten or added to. `passes` runs only the dQ kernel or only
@@ -257,8 +270,11 @@ def attn_bwd_step(q, k, v, dout, lse, delta, softmax_scale: float, causal: bool,
     a.stream = stream_ptr(q.device)
     share = {_lib.SPA_BWD_BOTH: 2.5, _lib.SPA_BWD_DQ_ONLY: 1.0, _lib.SPA_BWD_DKV_ONLY: 1.5}[a.passes]
     name = {_lib.SPA_BWD_BOTH: "bwd", _lib.SPA_BWD_DQ_ONLY: "bwd_dq", _lib.SPA_BWD_DKV_ONLY: "bwd_dkv"}[a.passes]
-    with _Timed(name, q.device, share * attn_flops(B, Sq, Sk, Hq, D, causal, causal_off)):
-        check(lib.spa_attn_bwd(C.byref(a)), "spa_attn_bwd")
+    with _Timed(name, q.device, share * _call_flops(B, Sq, Sk, Hq, D, causal, causal_off, seqs)):
+        if seqs is None:
+            check(lib.spa_attn_bwd(C.byref(a)), "spa_attn_bwd")
+        else:
+            check(lib.spa_attn_varlen_bwd(C.byref(a), _lib.seq_table(seqs), len(seqs)), "spa_attn_varlen_bwd")
 
 
 def cast_from_f32(src: torch.Tensor, dtype: torch.dtype, alpha: float = 1.0,
@@ -296,6 +312,33 @@ def flash_attn_backward(dout, q, k, v, out, lse, softmax_scale: Optional[float] 
     # each dq row, dk row and dv row has one owning CTA: no accumulator, nothing to zero
     attn_bwd_step(q, k, v, dout, lse, delta, softmax_scale, causal, None, dk, dv,
                   dq=dq, dq_overwrite=True, deterministic=deterministic)
+    return dq, dk, dv
+
+
+def packed_forward(q, k, v, seqs, softmax_scale: float, causal: bool):
+    """Attention over sequences packed in q, k, v [tokens, H, D]; `seqs` as in attn_fwd_step.
+    Returns (out [Tq,Hq,D], lse [Hq,Tq] fp32); every query row must belong to a sequence."""
+    Tq, Hq, _ = q.shape
+    out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    lse = torch.empty((Hq, Tq), dtype=torch.float32, device=q.device)
+    attn_fwd_step(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), softmax_scale, causal,
+                  lse.unsqueeze(0), out=out.unsqueeze(0), seqs=seqs)
+    return out, lse
+
+
+def packed_backward(dout, q, k, v, out, lse, seqs, softmax_scale: float, causal: bool,
+                    deterministic: bool = False, k_slice: slice = slice(None)):
+    """Gradients of packed_forward(q, k[k_slice], v[k_slice], ...): dq, dk, dv in q.dtype, rows
+    of k and v that no sequence uses get zeros."""
+    delta = bwd_delta(out.unsqueeze(0), dout.unsqueeze(0))
+    dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    all_keys = sum(s[3] for s in seqs) == k.shape[0]
+    dk, dv = [(torch.empty if all_keys else torch.zeros)(k.shape, dtype=k.dtype, device=k.device)
+              for _ in range(2)]
+    attn_bwd_step(q.unsqueeze(0), k[k_slice].unsqueeze(0), v[k_slice].unsqueeze(0), dout.unsqueeze(0),
+                  lse.unsqueeze(0), delta, softmax_scale, causal, None, dk[k_slice].unsqueeze(0),
+                  dv[k_slice].unsqueeze(0), dq=dq.unsqueeze(0), dq_overwrite=True,
+                  deterministic=deterministic, seqs=seqs)
     return dq, dk, dv
 
 

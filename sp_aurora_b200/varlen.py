@@ -11,8 +11,9 @@ Here they exist with flash-attn's varlen calling convention:
 Every sequence is sharded over the ring like a batch-1 tensor: rank r holds its r-th contiguous
 chunk (`*_varlen_func`), or, in the zigzag layout, its half-chunks r and 2W-1-r back to back
 (`zigzag_*`; the layout the balanced causal ring uses internally, here chosen by the caller, which
-saves the two re-layout exchanges). Each sequence runs as its own ring over views of the packed
-tensors (no copies; one set of kernel launches per sequence), so sequences never see each other.
+saves the two re-layout exchanges). On one rank all sequences go through one set of kernel
+launches (spa_attn_varlen_fwd / _bwd). On several each sequence runs as its own ring over views of
+the packed tensors (no copies; one set of launches per sequence). Sequences never see each other.
 """
 from __future__ import annotations
 
@@ -42,6 +43,41 @@ def _check_packed(q, k, v):
             raise ValueError(f"{name} must be packed [total_tokens, H, D], got {tuple(t.shape)}")
 
 
+def _one_rank(group) -> bool:
+    return not (dist.is_available() and dist.is_initialized()) or dist.get_world_size(group) == 1
+
+
+class VarlenFlashAttnFunc(torch.autograd.Function):
+    """Packed sequences on one rank (both layouts are the plain order there); returns out, lse."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, seqs, softmax_scale, causal, deterministic):
+        if softmax_scale is None:
+            softmax_scale = q.shape[-1] ** (-0.5)
+        local_attn.check_qkv(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0))
+        out, lse = local_attn.packed_forward(q, k, v, seqs, softmax_scale, causal)
+        ctx.save_for_backward(q, k, v, out, lse)
+        ctx.seqs, ctx.softmax_scale, ctx.causal = seqs, softmax_scale, causal
+        ctx.deterministic = bool(deterministic)
+        return out, lse
+
+    @staticmethod
+    def backward(ctx, dout, _dlse):
+        if dout.stride(-1) != 1:
+            dout = dout.contiguous()
+        q, k, v, out, lse = ctx.saved_tensors
+        dq, dk, dv = local_attn.packed_backward(dout, q, k, v, out, lse, ctx.seqs, ctx.softmax_scale,
+                                                ctx.causal, ctx.deterministic)
+        _lib.maybe_check_status()
+        return dq, dk, dv, None, None, None, None
+
+
+def _packed_one_rank(q, k, v, bq, bk, softmax_scale, causal, deterministic, return_attn_probs):
+    seqs = [(a, b - a, c, d - c, 0) for a, b, c, d in zip(bq, bq[1:], bk, bk[1:]) if b > a]
+    out, lse = VarlenFlashAttnFunc.apply(q, k, v, seqs, softmax_scale, causal, deterministic)
+    return (out, lse, None) if return_attn_probs else out
+
+
 def ring_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k=None, max_seqlen_q=None,
                                 max_seqlen_k=None, dropout_p=0.0, softmax_scale=None, causal=False,
                                 window_size=(-1, -1), alibi_slopes=None, deterministic=False,
@@ -55,6 +91,8 @@ def ring_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k=None, max_se
     bq, bk = _bounds(cu_seqlens_q, q.shape[0]), _bounds(cu_k, k.shape[0])
     if len(bq) != len(bk):
         raise ValueError("cu_seqlens_q and cu_seqlens_k describe different numbers of sequences")
+    if bq[-1] > 0 and _one_rank(group):
+        return _packed_one_rank(q, k, v, bq, bk, softmax_scale, causal, deterministic, return_attn_probs)
     outs, lses = [], []
     for i in range(len(bq) - 1):
         qi, ki, vi = q[bq[i]:bq[i + 1]], k[bk[i]:bk[i + 1]], v[bk[i]:bk[i + 1]]
@@ -134,6 +172,8 @@ def zigzag_ring_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k=None,
     bq, bk = _bounds(cu_seqlens_q, q.shape[0]), _bounds(cu_k, k.shape[0])
     if bq != bk:
         raise ValueError("the zigzag layout needs equal query and key lengths per sequence")
+    if bq[-1] > 0 and _one_rank(group):
+        return _packed_one_rank(q, k, v, bq, bk, softmax_scale, True, deterministic, return_attn_probs)
     outs, lses = [], []
     for i in range(len(bq) - 1):
         if bq[i + 1] == bq[i]:
