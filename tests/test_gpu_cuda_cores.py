@@ -1,0 +1,43 @@
+"""Tile edges of the CUDA-core kernels (64-row tiles, 4 or 8 rows per thread)."""
+import pytest
+import torch
+
+from oracle import attention_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (63, 65), (64, 64), (65, 129), (200, 130)])
+@pytest.mark.parametrize("D,causal,off", [(32, True, 0), (64, True, -70), (128, False, 0), (128, True, 60)])
+def test_fp32_tiles_match_the_oracle(Sq, Sk, D, causal, off):
+    """fp32 sums of at most 200 terms of unit size: 1e-5 is a hundred roundings."""
+    import sp_aurora_b200 as spa
+    from sp_aurora_b200 import local_attn as la
+    B, Hq, Hkv = 2, 4, 2
+    g = torch.Generator().manual_seed(5)
+    q, do = (torch.randn(B, Sq, Hq, D, generator=g) for _ in range(2))
+    kv = torch.randn(B, Sk, 2, Hkv, D, generator=g)
+    qc, doc, kvc = q.cuda(), do.cuda(), kv.cuda()
+    kc, vc = kvc[:, :, 0], kvc[:, :, 1]
+    scale = D ** -0.5
+    out, lse = torch.empty_like(qc), torch.empty(B, Hq, Sq, device="cuda")
+    la.attn_fwd_step(qc, kc, vc, scale, causal, lse, out=out, causal_off=off)
+    dq, dkv = torch.empty_like(qc), torch.empty_like(kvc)
+    la.attn_bwd_step(qc, kc, vc, doc, lse, la.bwd_delta(out, doc), scale, causal, None, dkv[:, :, 0], dkv[:, :, 1],
+                     causal_off=off, dq=dq, dq_overwrite=True)
+    spa.check_status()
+    # plain reference in 64 bits, rows without a visible key give zeros
+    qd, kd, vd, dd = (t.double().transpose(1, 2) for t in (q, kv[:, :, 0], kv[:, :, 1], do))
+    kd, vd = (t.repeat_interleave(Hq // Hkv, 1) for t in (kd, vd))
+    qd, kd, vd = (t.requires_grad_(True) for t in (qd, kd, vd))
+    s = scale * qd @ kd.transpose(2, 3)
+    seen = torch.ones(Sq, Sk, dtype=torch.bool)
+    if causal:
+        seen = torch.arange(Sk)[None] <= torch.arange(Sq)[:, None] + off
+    any_key = seen.any(1)[:, None]
+    p = torch.softmax(s.masked_fill(~seen & any_key, -torch.inf), -1) * any_key
+    o = p @ vd
+    gq, gk, gv = torch.autograd.grad(o, (qd, kd, vd), dd)
+    gk, gv = (t.view(B, Hkv, Hq // Hkv, Sk, D).sum(2) for t in (gk, gv))
+    for got, want in ((out, o), (dq, gq), (dkv[:, :, 0], gk), (dkv[:, :, 1], gv)):
+        assert (got.cpu().double().transpose(1, 2) - want).abs().max() <= 1e-5 * max(1.0, want.abs().max().item())
