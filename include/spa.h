@@ -73,6 +73,17 @@ typedef struct spa_fwd_args {
 int spa_attn_fwd(const spa_fwd_args* args);
 
 /*
+ * The same call with scratch memory. Problems whose query blocks do not fill the GPU (a short
+ * block of queries over a long context) split the keys of a block between several CTAs and
+ * join the partial results; spa_attn_fwd_workspace says how many bytes that takes (0: this
+ * problem is not split; negative: an SPA_E* code), spa_attn_fwd_ws uses them (16-byte
+ * aligned, contents undefined afterwards, per call: calls that overlap need their own). A null
+ * workspace is spa_attn_fwd.
+ */
+int64_t spa_attn_fwd_workspace(const spa_fwd_args* args);
+int spa_attn_fwd_ws(const spa_fwd_args* args, void* workspace, int64_t bytes);
+
+/*
  * delta[b,h,s] = sum_d dout[b,s,h,d] * out[b,s,h,d]  (fp32), the row term of
  * the softmax backward. No reference counterpart as a separate function: the
  * reference obtains it implicitly through autograd

@@ -91,6 +91,8 @@ class Seq(C.Structure):
 _I64x4 = C.c_int64 * 4
 _SIGNATURES = {
     "spa_attn_fwd": (C.c_int, [C.POINTER(FwdArgs)]),
+    "spa_attn_fwd_workspace": (C.c_int64, [C.POINTER(FwdArgs)]),
+    "spa_attn_fwd_ws": (C.c_int, [C.POINTER(FwdArgs), C.c_void_p, C.c_int64]),
     "spa_attn_bwd": (C.c_int, [C.POINTER(BwdArgs)]),
     "spa_attn_varlen_fwd": (C.c_int, [C.POINTER(FwdArgs), C.POINTER(Seq), C.c_int32]),
     "spa_attn_varlen_bwd": (C.c_int, [C.POINTER(BwdArgs), C.POINTER(Seq), C.c_int32]),

@@ -21,6 +21,7 @@
 #include <cuda_fp16.h>
 #include <math.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "spa_internal.h"
@@ -43,6 +44,9 @@ struct FwdParams {
   int causal, causal_off, merge_prev;
   int n_qblk;
   int chunk;   // query blocks per scheduling chunk (n_qblk or 1)
+  int row_step, head_step;   // tile 1 of a CTA = tile 0 + so many query rows and heads
+  int split;   // CTAs sharing the keys of a block; > 1: partial results go to `part`
+  float* part;               // [split][B][Sq][Hq][D] normalised outputs, then [split][B][Hq][Sq] lse
   float scale_log2;
   void* out;
   int64_t o_sb, o_ss, o_sh;
@@ -77,14 +81,20 @@ __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// kVar: one launch over the sequences of a packed batch (B = 1). tm_q and tm_k then cover the
-// whole packed tensors, the V map comes from the sequence's table entry (see varlen.cuh).
-template <int D, typename T, bool kVar>
+// How the work of a launch is laid out. kPlain: a CTA owns two adjacent query tiles of a head and
+// all their keys. kVarlen: the same over the sequences of a packed batch (B = 1); tm_q and tm_k
+// then cover the whole packed tensors, the V map comes from the sequence's table entry (see
+// varlen.cuh). kCut: short grids, see plan_fwd. Instances apart, because the extra address
+// arithmetic of the other two costs the plain one 2-3 % (S=16384, 16 heads: 979 -> 1006 us).
+enum FwdMode { kPlain, kVarlen, kCut };
+
+template <int D, typename T, FwdMode kMode>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
                       const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const FwdParams p,
-                      const __grid_constant__ VarTable<kVar, 1> var) {
+                      const __grid_constant__ VarTable<kMode == kVarlen, 1> var) {
+  constexpr bool kVar = kMode == kVarlen;
   using L = FwdSmem<D>;
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   extern __shared__ uint8_t smem_raw[];
@@ -104,23 +114,30 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  // Work decode: query blocks of one chunk fastest (longest first under a causal mask),
-  // then heads, batch, chunks. The host picks the chunk: all query blocks (CTAs resident
-  // together then stream the K/V of one kv head, which stays in L2: S=131072 causal
-  // 993 -> 1036 TFLOP/s), or one block for small causal problems, where
+  // Work decode: key slices of a block fastest, then query blocks of one chunk (longest first
+  // under a causal mask), then heads, batch, chunks. The host picks the chunk: all query
+  // blocks (CTAs resident together then stream the K/V of one kv head, which stays in L2:
+  // S=131072 causal 993 -> 1036 TFLOP/s), or one block for small causal problems, where
   // longest-block-first over all heads matters more. Packed sequences: heads fastest, then
   // the blocks of all sequences by falling distance from the start of their sequence.
+  const int row_step = kMode == kCut ? p.row_step : kTileM;
+  const int head_step = kMode == kCut ? p.head_step : 0;
   int w = blockIdx.x;
-  int h, b, qblk, sg = 0;
+  int h, b, qblk, sg = 0, ks = 0;
   if constexpr (kVar) {
     h = w % p.Hq;
     b = 0;
     qblk = var.decode(w / p.Hq, sg);
   } else {
+    if constexpr (kMode == kCut) {
+      ks = w % p.split;
+      w /= p.split;
+    }
     const int q_lo = w % p.chunk;
     w /= p.chunk;
-    h = w % p.Hq;
-    w /= p.Hq;
+    const int n_heads = p.Hq >> head_step;
+    h = (w % n_heads) << head_step;
+    w /= n_heads;
     b = w % p.B;
     qblk = p.n_qblk - 1 - ((w / p.B) * p.chunk + q_lo);
   }
@@ -131,13 +148,13 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int k_row0 = kVar ? var.seq(sg).k0 : 0;
   const CUtensorMap* const v_map = kVar ? var.map(sg, 0) : &tm_v;
   const int hk = h / (p.Hq / p.Hkv);
-  const int q0 = qblk * 2 * kTileM;
+  const int q0 = qblk * (kTileM + row_step);
 
   // Number of K/V tiles each query tile attends to.
   int n_t[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int r0 = q0 + t * kTileM;
+    const int r0 = q0 + t * row_step;
     int n = 0;
     if (r0 < Sq) {
       n = (Sk + kTileN - 1) / kTileN;
@@ -149,6 +166,15 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
     }
     n_t[t] = n;
+  }
+  int key_base = 0;   // first key of this CTA's slice
+  if (kMode == kCut && p.split > 1) {
+    const int n_all = max(n_t[0], n_t[1]);
+    const int lo = (int)((long long)n_all * ks / p.split);
+    const int hi = (int)((long long)n_all * (ks + 1) / p.split);
+    n_t[0] = max(0, min(n_t[0], hi) - lo);
+    n_t[1] = max(0, min(n_t[1], hi) - lo);
+    key_base = lo * kTileN;
   }
   const int nmax = max(n_t[0], n_t[1]);
 
@@ -183,12 +209,12 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(v_map);
-      const int q_tiles = (n_t[1] > 0 || q0 + kTileM < Sq) ? 2 : 1;
+      const int q_tiles = (n_t[1] > 0 || q0 + row_step < Sq) ? 2 : 1;
       mbar_arrive_expect_tx(q_full, q_tiles * L::kTileBytes);
       for (int t = 0; t < q_tiles; ++t)
         for (int s = 0; s < D / 64; ++s)
           tma_load_4d(smem + L::kQOff + t * L::kTileBytes + s * L::kSlabBytes, &tm_q, q_full,
-                      s * 64, q_row0 + q0 + t * kTileM, h, b);
+                      s * 64, q_row0 + q0 + t * row_step, h + t * head_step, b);
       const int nfill = 2 * nmax;
       for (int n = 0; n < nfill; ++n) {
         const int slot = n % L::kStages;
@@ -197,7 +223,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
         mbar_arrive_expect_tx(&kv_full[slot], L::kTileBytes);
         const CUtensorMap* tm = (n & 1) ? v_map : &tm_k;
         const int j = n >> 1;
-        const int row = j * kTileN + ((n & 1) ? 0 : k_row0);
+        const int row = key_base + j * kTileN + ((n & 1) ? 0 : k_row0);
         for (int s = 0; s < D / 64; ++s)
           tma_load_4d(smem + L::kKVOff + slot * L::kTileBytes + s * L::kSlabBytes, tm,
                       &kv_full[slot], s * 64, row, hk, b);
@@ -284,12 +310,13 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
     const int t = warp >> 2;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
-    const int qrow = q0 + t * kTileM + row_in_tile;
+    const int qrow = q0 + t * row_step + row_in_tile;
+    const int hq = h + t * head_step;
     const uint32_t lane_field = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t tmem_s = tmem_base + lane_field + t * 128;
     const uint32_t tmem_o = tmem_base + lane_field + 256 + t * D;
     const int nt = n_t[t];
-    const int tile_row_min = q0 + t * kTileM;
+    const int tile_row_min = q0 + t * row_step;
     const float ninf = -INFINITY;
 
     float m_used = ninf;
@@ -306,7 +333,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       tmem_ld_wait();
       float* s = reinterpret_cast<float*>(sr);
 
-      const int k0 = j * kTileN;
+      const int k0 = key_base + j * kTileN;
       const bool need_mask = (k0 + kTileN > Sk) ||
                              (p.causal && ((long long)k0 + kTileN - 1 >
                                            (long long)tile_row_min + causal_off));
@@ -381,7 +408,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       const bool have = (nt > 0) && (l > 0.f);
       const float inv_l = have ? 1.f / l : 0.f;
       const float lse_blk = have ? (m_used + log2f(l)) * kLn2 : ninf;
-      const size_t lse_idx = (size_t)b * p.lse_sb + (size_t)h * p.lse_sh + q_row0 + qrow;
+      const size_t lse_idx = (size_t)b * p.lse_sb + (size_t)hq * p.lse_sh + q_row0 + qrow;
       float w_old = 0.f, w_blk = have ? 1.f : 0.f, lse_new = lse_blk;
       if (p.merge_prev && row_ok) {
         const float lse_old = p.lse[lse_idx];
@@ -399,12 +426,19 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
           w_blk = e_blk / sum;
         }
       }
-      if (row_ok) p.lse[lse_idx] = lse_new;
+      const bool partial = kMode == kCut && p.split > 1;
+      if (row_ok) {
+        if (partial)   // a NaN row must not look like a slice without visible keys
+          p.part[(size_t)p.split * p.B * p.Sq * p.Hq * D + (((size_t)ks * p.B + b) * p.Hq + hq) * p.Sq + qrow] =
+              nt > 0 && l != l ? l : lse_new;
+        else
+          p.lse[lse_idx] = lse_new;
+      }
       const float o_scale = inv_l * w_blk;
-      float* acc_row =
-          p.out_acc ? p.out_acc + (((size_t)b * p.Sq + qrow) * p.Hq + h) * D : nullptr;
-      T* out_row = p.out ? reinterpret_cast<T*>(p.out) + (size_t)b * p.o_sb +
-                               (size_t)(q_row0 + qrow) * p.o_ss + (size_t)h * p.o_sh
+      float* acc_base = partial ? (nt > 0 ? p.part + (size_t)ks * p.B * p.Sq * p.Hq * D : nullptr) : p.out_acc;
+      float* acc_row = acc_base ? acc_base + (((size_t)b * p.Sq + qrow) * p.Hq + hq) * D : nullptr;
+      T* out_row = p.out && !partial ? reinterpret_cast<T*>(p.out) + (size_t)b * p.o_sb +
+                               (size_t)(q_row0 + qrow) * p.o_ss + (size_t)hq * p.o_sh
                          : nullptr;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
@@ -462,9 +496,89 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
 }
 
-template <int D, typename T, bool kVar>
-int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq) {
+// Joins the key slices of a split forward: out = sum_s w_s out_s / sum_s w_s with
+// w_s = exp(lse_s - max lse), lse = logsumexp. D/4 lanes per row, a row per lane group; the
+// partial results were written just before and are read from L2.
+template <int D, typename T>
+__global__ void __launch_bounds__(256)
+combine_splits_kernel(const FwdParams p) {
+  constexpr int kLanes = D / 4;
+  const long long n_rows = (long long)p.B * p.Sq * p.Hq;
+  const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  if (row >= n_rows) return;
+  const int c = (threadIdx.x % kLanes) * 4;
+  const int h = (int)(row % p.Hq);
+  const int q = (int)((row / p.Hq) % p.Sq);
+  const int b = (int)(row / ((long long)p.Hq * p.Sq));
+  const float* lse_part = p.part + (size_t)p.split * n_rows * D + ((size_t)b * p.Hq + h) * p.Sq + q;
+  const float* o_part = p.part + (size_t)row * D + c;
+  float mx = -INFINITY;
+  for (int s = 0; s < p.split; ++s) mx = fmaxf(mx, lse_part[(size_t)s * n_rows]);
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  float sum = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < p.split; ++s) {
+    const float ls = lse_part[(size_t)s * n_rows];
+    if (ls == -INFINITY) continue;   // no visible key in the slice: nothing was written
+    const float4 v = *reinterpret_cast<const float4*>(o_part + (size_t)s * n_rows * D);
+    const float w = expf(ls - mx);
+    sum += w;
+    o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
+  }
+  const float inv = sum > 0.f ? 1.f / sum : 0.f;
+  if (c == 0) p.lse[(size_t)b * p.lse_sb + (size_t)h * p.lse_sh + q] = sum > 0.f ? mx + logf(sum) : -INFINITY;
+  T* dst = reinterpret_cast<T*>(p.out) + (size_t)b * p.o_sb + (size_t)q * p.o_ss + (size_t)h * p.o_sh + c;
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(o.x * inv, o.y * inv), pack2<T>(o.z * inv, o.w * inv));
+}
+
+struct FwdPlan {
+  bool pair_heads;   // the two tiles of a CTA are one query tile of two heads of a kv group
+  int split;
+};
+
+// How a plain forward is cut. A query-tile count that is odd leaves half of a CTA's ping-pong
+// idle in the last block (all of it when there is one tile): with an even number of heads per
+// kv head the tiles of two heads are paired instead. If the grid is still smaller than the
+// chip, or one causal block outlasts everything else, the keys of each block are cut into
+// `split` slices whose partial results a second kernel joins. `workspace` false: no splitting.
+// 128 queries of 32 / 8 heads over 16384 keys, batch 2, D=128: 250 -> 95 us; 40 queries of 8 heads over 8000 keys: 119 -> 28; 4096 causal rows of 4 heads: 76 -> 54.
+// Times are in units of one key tile of both query tiles (2.2 us).
+FwdPlan plan_fwd(const spa_fwd_args* a, bool workspace) {
+  FwdPlan plan{false, 1};
+  const int tiles = ceil_div(a->Sq, kTileM);
+  plan.pair_heads = tiles % 2 == 1 && tiles <= 5 && (a->Hq / a->Hkv) % 2 == 0;
+  if (!workspace || a->merge_prev || a->out_acc) return plan;
+  const long long blocks = plan.pair_heads ? (long long)tiles * (a->Hq / 2) * a->B
+                                           : (long long)ceil_div(tiles, 2) * a->Hq * a->B;
+  const int n_sm = device_sm_count();
+  if (blocks >= 2ll * n_sm) return plan;
+  long long longest = ceil_div(a->Sk, kTileN);
+  if (a->causal)
+    longest = std::max(0ll, std::min(longest, ((long long)a->Sq - 1 + a->causal_off) / kTileN + 1));
+  const double mean = a->causal && a->causal_off < a->Sk ? 0.5 * (longest + 1) : (double)longest;
+  const double fill = 1.5;             // prologue and epilogue of a CTA
+  const double rows = (double)a->B * a->Sq * a->Hq;
+  double best = 0.0;
+  for (int s = 1; s <= 16; ++s) {
+    if (s > 1 && longest / s < 4) break;
+    const double waves = (double)((blocks * s + n_sm - 1) / n_sm);
+    const double work = blocks * s * (mean / s + fill) / n_sm;
+    const double step = longest / (double)s + fill;
+    double t = a->causal ? std::max(step, work) : waves * step;
+    if (s > 1) t += 2.5 + s * rows * a->D * 8.0 / 1e7;   // join: a launch, and its bytes through L2
+    if (s == 1 || t < best * 0.93) {
+      best = t;
+      plan.split = s;
+    }
+  }
+  return plan;
+}
+
+template <int D, typename T, FwdMode kMode>
+int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq, const FwdPlan& plan,
+                     float* part) {
   using L = FwdSmem<D>;
+  constexpr bool kVar = kMode == kVarlen;
   CUtensorMap tq, tk, tv;
   if (encode_rows_map(&tq, a->q, is_bf16, D, a->Sq, a->Hq, a->B, a->q_ss, a->q_sh, a->q_sb, kTileM))
     return SPA_ECUDA;
@@ -475,7 +589,11 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, in
   FwdParams p;
   p.B = a->B; p.Sq = a->Sq; p.Sk = a->Sk; p.Hq = a->Hq; p.Hkv = a->Hkv;
   p.causal = a->causal; p.causal_off = a->causal_off; p.merge_prev = a->merge_prev;
-  p.n_qblk = ceil_div(a->Sq, 2 * kTileM);
+  p.row_step = plan.pair_heads ? 0 : kTileM;
+  p.head_step = plan.pair_heads ? 1 : 0;
+  p.split = plan.split;
+  p.part = part;
+  p.n_qblk = ceil_div(a->Sq, kTileM + p.row_step);
   p.chunk = (!a->causal || p.n_qblk >= 256) ? p.n_qblk : 1;
   p.scale_log2 = a->scale * kLog2e;
   p.out = a->out; p.o_sb = a->o_sb; p.o_ss = a->o_ss; p.o_sh = a->o_sh;
@@ -483,10 +601,10 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, in
   p.status = device_status_word();
   if (!p.status) return SPA_ECUDA;
   const int smem_bytes = L::kTotal + 1024;
-  auto kern = attn_fwd_sm100_kernel<D, T, kVar>;
+  auto kern = attn_fwd_sm100_kernel<D, T, kMode>;
   int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, "fwd sm100");
   if (rc) return rc;
-  long long grid = (long long)p.n_qblk * a->B * a->Hq;
+  long long grid = (long long)p.n_qblk * a->B * (a->Hq >> p.head_step) * p.split;
   VarTable<kVar, 1> var;
   if constexpr (kVar) {
     grid = fill_var_table(&var, seqs, n_seq, 2 * kTileM, /*by_key=*/false) * a->Hq;
@@ -502,6 +620,10 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, in
     return SPA_EINVAL;
   }
   kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, p, var);
+  if (kMode == kCut && p.split > 1) {
+    const long long threads = (long long)a->B * a->Sq * a->Hq * (D / 4);
+    combine_splits_kernel<D, T><<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)a->stream>>>(p);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("fwd sm100 launch: %s", cudaGetErrorString(e));
@@ -510,15 +632,15 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, in
   return SPA_OK;
 }
 
-template <bool kVar>
-int launch_fwd_any(const spa_fwd_args* a, const spa_seq* seqs, int n_seq) {
+template <FwdMode kMode>
+int launch_fwd_any(const spa_fwd_args* a, const spa_seq* seqs, int n_seq, const FwdPlan& plan, float* part) {
   const bool bf = a->dtype == SPA_DTYPE_BF16;
   if (a->D == 128) {
-    return bf ? launch_fwd_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
-              : launch_fwd_typed<128, __half, kVar>(a, 0, seqs, n_seq);
+    return bf ? launch_fwd_typed<128, __nv_bfloat16, kMode>(a, 1, seqs, n_seq, plan, part)
+              : launch_fwd_typed<128, __half, kMode>(a, 0, seqs, n_seq, plan, part);
   } else if (a->D == 64) {
-    return bf ? launch_fwd_typed<64, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
-              : launch_fwd_typed<64, __half, kVar>(a, 0, seqs, n_seq);
+    return bf ? launch_fwd_typed<64, __nv_bfloat16, kMode>(a, 1, seqs, n_seq, plan, part)
+              : launch_fwd_typed<64, __half, kMode>(a, 0, seqs, n_seq, plan, part);
   }
   set_error("tensor-core forward supports head_dim 64 and 128, got %d", a->D);
   return SPA_EUNSUPPORTED;
@@ -526,10 +648,19 @@ int launch_fwd_any(const spa_fwd_args* a, const spa_seq* seqs, int n_seq) {
 
 }  // namespace
 
-int launch_fwd_sm100(const spa_fwd_args* a) { return launch_fwd_any<false>(a, nullptr, 0); }
+int64_t fwd_sm100_workspace(const spa_fwd_args* a) {
+  const FwdPlan plan = plan_fwd(a, true);
+  return plan.split == 1 ? 0 : (int64_t)plan.split * a->B * a->Sq * a->Hq * (a->D + 1) * (int64_t)sizeof(float);
+}
+
+int launch_fwd_sm100(const spa_fwd_args* a, float* workspace) {
+  const FwdPlan plan = plan_fwd(a, workspace != nullptr);
+  return plan.pair_heads || plan.split > 1 ? launch_fwd_any<kCut>(a, nullptr, 0, plan, workspace)
+                                           : launch_fwd_any<kPlain>(a, nullptr, 0, plan, nullptr);
+}
 
 int launch_fwd_sm100_var(const spa_fwd_args* a, const spa_seq* seqs, int n_seq) {
-  return launch_fwd_any<true>(a, seqs, n_seq);
+  return launch_fwd_any<kVarlen>(a, seqs, n_seq, FwdPlan{false, 1}, nullptr);
 }
 
 }  // namespace spa

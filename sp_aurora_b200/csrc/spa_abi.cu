@@ -777,14 +777,34 @@ static int prepare_fwd(const spa_fwd_args* args, spa_fwd_args* n, const char* wh
 
 static bool on_tensor_cores(int dtype, int D) { return dtype != SPA_DTYPE_F32 && D != 32 && !force_simt(); }
 
-int spa_attn_fwd(const spa_fwd_args* args) {
+int64_t spa_attn_fwd_workspace(const spa_fwd_args* args) {
+  spa_fwd_args n;
+  const int rc = prepare_fwd(args, &n, "spa_attn_fwd_workspace");
+  if (rc) return rc;
+  return on_tensor_cores(n.dtype, n.D) ? fwd_sm100_workspace(&n) : 0;
+}
+
+int spa_attn_fwd_ws(const spa_fwd_args* args, void* workspace, int64_t bytes) {
   spa_fwd_args n;
   int rc = prepare_fwd(args, &n, "spa_attn_fwd");
   if (rc) return rc;
-  rc = on_tensor_cores(n.dtype, n.D) ? launch_fwd_sm100(&n) : launch_fwd_simt(&n);
-  if (rc == SPA_OK) note_launch(1);
+  if (!on_tensor_cores(n.dtype, n.D)) {
+    rc = launch_fwd_simt(&n);
+    if (rc == SPA_OK) note_launch(1);
+    return rc;
+  }
+  const int64_t need = workspace ? fwd_sm100_workspace(&n) : 0;
+  if (need > bytes || ((uintptr_t)workspace & 15)) {
+    set_error("spa_attn_fwd: workspace of %lld bytes (16-byte aligned) needed, got %lld", (long long)need,
+              (long long)bytes);
+    return SPA_EINVAL;
+  }
+  rc = launch_fwd_sm100(&n, static_cast<float*>(workspace));
+  if (rc == SPA_OK) note_launch(need > 0 ? 2 : 1);
   return rc;
 }
+
+int spa_attn_fwd(const spa_fwd_args* args) { return spa_attn_fwd_ws(args, nullptr, 0); }
 
 static int validate_seqs(const spa_seq* seqs, int n, int B, int Sq, int Sk, const char* what) {
   if (!seqs || n <= 0 || B != 1) {

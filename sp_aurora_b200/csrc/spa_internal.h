@@ -40,7 +40,10 @@ int device_sm_count();
 
 // Launchers (return a spa status code). Arguments arrive normalised: zero stride
 // triples of spa.h are already replaced by the contiguous strides.
-int launch_fwd_sm100(const spa_fwd_args* a);
+// `workspace` (may be null: then the keys of a block are never split between CTAs) holds
+// fwd_sm100_workspace(a) bytes, 16-byte aligned.
+int64_t fwd_sm100_workspace(const spa_fwd_args* a);
+int launch_fwd_sm100(const spa_fwd_args* a, float* workspace);
 int launch_bwd_dq_sm100(const spa_bwd_args* a);       // query-stationary pass: dQ
 int launch_bwd_dkv_sm100(const spa_bwd_args* a);      // K/V-stationary pass: dK, dV
 // The same kernels over up to kVarMaxSeqs sequences of a packed batch (B = 1).

@@ -178,7 +178,12 @@ def attn_fwd_step(q, k, v, softmax_scale: float, causal: bool, lse: torch.Tensor
     a.stream = stream_ptr(q.device)
     with _Timed("fwd", q.device, _call_flops(B, Sq, Sk, Hq, D, causal, causal_off, seqs)):
         if seqs is None:
-            check(lib.spa_attn_fwd(C.byref(a)), "spa_attn_fwd")
+            need = lib.spa_attn_fwd_workspace(C.byref(a))
+            if need > 0:    # short grid: the keys are split between CTAs
+                ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+                check(lib.spa_attn_fwd_ws(C.byref(a), ws.data_ptr(), need), "spa_attn_fwd")
+            else:
+                check(lib.spa_attn_fwd(C.byref(a)), "spa_attn_fwd")
         else:
             check(lib.spa_attn_varlen_fwd(C.byref(a), _lib.seq_table(seqs), len(seqs)), "spa_attn_varlen_fwd")
 
