@@ -7,11 +7,12 @@
 // triu(diagonal=1) mask, lse = logsumexp, out = softmax*V) and the merge follows
 // sp_aurora/utils.py:99-104.
 //
-// CTA = 10 warps:
+// CTA = 12 warps:
 //   warps 0-3  softmax group of query tile 0 (thread = one query row)
 //   warps 4-7  softmax group of query tile 1
 //   warp  8    TMA producer (lane 0)
 //   warp  9    tcgen05.mma issuer (lane 0); also owns the TMEM allocation
+//   warps 10, 11 complete the warpgroup that gives registers to the softmax groups
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
 // The probabilities P (bf16/fp16, two per 32-bit column) overwrite the first 64
 // columns of their S tile and feed the PV MMA as operand A straight from TMEM:
@@ -34,7 +35,15 @@ namespace {
 
 constexpr int kTileM = 128;          // query rows per tile
 constexpr int kTileN = 128;          // keys per K/V tile
-constexpr int kThreads = 320;
+constexpr int kThreads = 384;
+// Registers: 384 threads are launched with 168 each, and a softmax thread wants its 128 scores and
+// 64 packed probabilities at once: at 168 the loop spilled 76 to 130 bytes. The third warpgroup
+// gives up what the other two take: 2 * 128 * 208 + 128 * 88 = 384 * 168. (With 320 threads the
+// cap is 168 as well: registers are handed out per scheduler, and two of them have three warps.)
+// Causal, D=128: 3001 rows x 2 of 32 heads 192 -> 185 us, 8192 rows 525 -> 513, 16384 rows of 16
+// heads 992 -> 958.
+constexpr int kSoftmaxRegs = 208, kIssueRegs = 88;
+static_assert(2 * 128 * kSoftmaxRegs + 128 * kIssueRegs <= kThreads * 168, "register split");
 constexpr float kRescaleThreshold = 8.0f;  // in log2 units
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -203,7 +212,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wc{p.status, cta_abort};
 
-  if (warp == 8) {
+  if (warp >= 8) {
+    reg_shrink<kIssueRegs>();
+    if (warp == 8) {
     // ------------------------------------------------------------------ TMA
     if (lane == 0 && nmax > 0) {
       tma_prefetch_desc(&tm_q);
@@ -229,7 +240,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
                       &kv_full[slot], s * 64, row, hk, b);
       }
     }
-  } else if (warp == 9) {
+    } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA
     // One elected lane issues every MMA (measured faster than predicated
     // warp-uniform issue); descriptors are precomputed, offsets are constants.
@@ -305,8 +316,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
       }
     }
+    }
   } else {
     // -------------------------------------------------------------- softmax
+    reg_grow<kSoftmaxRegs>();
     const int t = warp >> 2;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;

@@ -61,6 +61,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Hand registers from one warpgroup to another (every warp of the warpgroup must get here). What
+// the growing warpgroups take has to be given up by the others: the block owns what it was
+// launched with.
+template <int kRegs>
+__device__ __forceinline__ void reg_grow() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void reg_shrink() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+
 // Per-CTA view of the abort machinery.
 struct WaitCtx {
   int* status;            // global status word (4 ints)
