@@ -131,7 +131,7 @@ def _rebuild_if_stale() -> str:
         return ""
     try:
         stale = _build._stale(_LIB_PATH, [_build.CSRC / s for s in _build.SOURCES] + _build.HEADERS)
-        if stale:
+        if stale or _build._stale(_build.NATIVE_PATH, _build.NATIVE_DEPS):
             _build.build()      # serialised across processes by a file lock; re-checks staleness
     except RuntimeError as e:
         return str(e)

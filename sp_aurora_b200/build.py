@@ -1,4 +1,5 @@
-"""Build libspaurora_sm100.so (the C-ABI CUDA library) in-tree with nvcc.
+"""Build libspaurora_sm100.so (the C-ABI CUDA library, nvcc) and _native.so (the C++ autograd node
+of the one-rank calls, g++ against the installed torch) in-tree.
 
     python -m sp_aurora_b200.build [--force]
 
@@ -28,6 +29,11 @@ NVCC_FLAGS = [
     "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
     "-Xcompiler", "-fPIC", "--use_fast_math=false", "-cudart", "static",
 ]
+
+
+NATIVE_PATH = PKG_DIR / "_native.so"
+NATIVE_SOURCE = CSRC / "native_path.cpp"
+NATIVE_DEPS = [NATIVE_SOURCE, PKG_DIR.parent / "include" / "spa.h"]
 
 
 def _nvcc() -> str:
@@ -82,9 +88,13 @@ def _build_locked(force: bool, verbose: bool) -> Path:
             raise RuntimeError(f"nvcc failed for {s.name}:\n{r.stdout}\n{r.stderr}")
         return o
 
-    if jobs:
-        with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 1)) as ex:
+    native = force or _stale(NATIVE_PATH, NATIVE_DEPS)
+    if jobs or native:
+        with ThreadPoolExecutor(max_workers=min(len(jobs) + 1, os.cpu_count() or 1)) as ex:
+            pending = ex.submit(_build_native, verbose) if native else None
             list(ex.map(compile_one, jobs))
+            if pending is not None:
+                pending.result()
     objs = [obj_dir / (src + ".o") for src in SOURCES]
     if force or jobs or _stale(LIB_PATH, objs):
         tmp = LIB_PATH.with_name(f"{LIB_PATH.name}.{os.getpid()}.tmp")
@@ -97,6 +107,27 @@ def _build_locked(force: bool, verbose: bool) -> Path:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, LIB_PATH)
     return LIB_PATH
+
+
+def _build_native(verbose: bool) -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [*cpp_extension.include_paths(), str(cuda / "include"), sysconfig.get_paths()["include"]]
+    lib_dir = Path(torch.__file__).resolve().parent / "lib"
+    tmp = NATIVE_PATH.with_name(f"{NATIVE_PATH.name}.{os.getpid()}.tmp")
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_native",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in includes], str(NATIVE_SOURCE), "-o", str(tmp), f"-L{lib_dir}",
+           *[f"-l{n}" for n in ("c10", "c10_cuda", "torch_cpu", "torch_cuda", "torch", "torch_python")]]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {NATIVE_SOURCE.name}:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, NATIVE_PATH)
 
 
 if __name__ == "__main__":

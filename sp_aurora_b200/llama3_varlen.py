@@ -31,7 +31,7 @@ from typing import Callable, List, Optional, Tuple
 import torch
 import torch.distributed as dist
 
-from . import _lib, local_attn
+from . import _lib, local_attn, native
 from .local_attn import check_unsupported_kwargs
 
 __all__ = ["llama3_flash_attn_prepare_cu_seqlens", "llama3_flash_attn_varlen_func",
@@ -258,6 +258,20 @@ class Llama3FlashAttnVarlenFunc(torch.autograd.Function):
         return (dq, dk, dv) + (None,) * 9
 
 
+def _native_one_rank(q, k, v, cu_q, cu_k, heads_k_stride, k_slice, softmax_scale, causal, deterministic, group):
+    """(out, lse) through the one-rank node, or None for tables and arguments that need the
+    general path (which checks them again and words the errors)."""
+    if (dist.is_available() and dist.is_initialized() and dist.get_world_size(group) != 1) or \
+            (heads_k_stride and (int(heads_k_stride) <= 0 or k.shape[1] % int(heads_k_stride))):
+        return None
+    segs = _segments(cu_q, cu_k)
+    start, stop, step = k_slice.indices(k.shape[0])
+    if step != 1 or not _one_launch(segs, q.shape[0], stop - start) or segs[-1][1] != q.shape[0]:
+        return None
+    seqs = [(q0, sq, start + k0, sk, off) for q0, sq, k0, sk, off in _seqs(segs)]
+    return native.attention_packed(q, k, v, seqs, softmax_scale, causal, deterministic, group)
+
+
 def llama3_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q=None,
                                   max_seqlen_k=None, heads_k_stride: Optional[int] = None,
                                   local_k_slice: Optional[slice] = None, dropout_p=0.0,
@@ -278,6 +292,10 @@ def llama3_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqle
             raise ValueError(f"{name} must be packed [tokens, H, D], got {tuple(t.shape)}")
     if local_k_slice is None:
         raise ValueError("local_k_slice is required (llama3_flash_attn_prepare_cu_seqlens returns it)")
+    res = _native_one_rank(q, k, v, cu_seqlens_q, cu_seqlens_k, heads_k_stride, local_k_slice, softmax_scale,
+                           causal, deterministic, group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return Llama3FlashAttnVarlenFunc.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, heads_k_stride,
                                            local_k_slice, softmax_scale, causal, deterministic,
                                            return_attn_probs, group)

@@ -1,0 +1,66 @@
+"""One-rank attention through the C++ autograd node of `_native.so` (csrc/native_path.cpp).
+
+Every function answers (out, lse), or None where the call has to go the general way: several
+ranks, per-kernel timing, or arguments that the node does not take (the general way also words
+the errors)."""
+from __future__ import annotations
+
+import ctypes as C
+
+import torch.distributed as dist
+
+from . import _lib, local_attn
+
+try:
+    from . import _native
+except ImportError as e:
+    raise ImportError("_native.so is missing or was built against another torch: build it with "
+                      "`python sp_aurora_b200/build.py` (this package has no fallback path)") from e
+
+_native.set_api([C.cast(getattr(_lib.lib, name), C.c_void_p).value for name in (
+    "spa_attn_fwd", "spa_attn_fwd_workspace", "spa_attn_fwd_ws", "spa_attn_bwd", "spa_attn_varlen_fwd",
+    "spa_attn_varlen_bwd", "spa_bwd_delta", "spa_check_status", "spa_last_error")], _lib.SpaError)
+
+
+def _general(group) -> bool:
+    return local_attn.KERNEL_TIMERS is not None or (
+        dist.is_available() and dist.is_initialized() and dist.get_world_size(group) != 1)
+
+
+def _scale(s):
+    return None if s is None else float(s)
+
+
+def attention(q, k, v, softmax_scale, causal, deterministic=False, group=None):
+    """q, k, v [B,S,H,D]."""
+    if _general(group):
+        return None
+    return _native.attention(q, k, v, _scale(softmax_scale), bool(causal), bool(deterministic), False)
+
+
+def attention_local(q, k, v, softmax_scale, causal):
+    """The same on this rank alone, whatever the groups; lse is marked as non-differentiable."""
+    if local_attn.KERNEL_TIMERS is not None:
+        return None
+    return _native.attention(q, k, v, _scale(softmax_scale), bool(causal), False, True)
+
+
+def attention_kvpacked(q, kv, softmax_scale, causal, deterministic=False, group=None):
+    """kv [B,S,2,H,D]; its gradient is written in that layout."""
+    if _general(group):
+        return None
+    return _native.attention_kvpacked(q, kv, _scale(softmax_scale), bool(causal), bool(deterministic))
+
+
+def attention_qkvpacked(qkv, softmax_scale, causal, deterministic=False, group=None):
+    """qkv [B,S,3,H,D]; its gradient is written in that layout."""
+    if _general(group):
+        return None
+    return _native.attention_qkvpacked(qkv, _scale(softmax_scale), bool(causal), bool(deterministic))
+
+
+def attention_packed(q, k, v, seqs, softmax_scale, causal, deterministic=False, group=None):
+    """Packed sequences, q, k, v [tokens,H,D]; `seqs` as in local_attn.attn_fwd_step."""
+    if _general(group):
+        return None
+    return _native.attention_packed(q, k, v, seqs, _scale(softmax_scale), bool(causal), bool(deterministic))

@@ -25,7 +25,7 @@ import torch.distributed as dist
 
 import os
 
-from . import _lib, local_attn, zigzag
+from . import _lib, local_attn, native, zigzag
 from .local_attn import check_unsupported_kwargs
 
 __all__ = [
@@ -286,6 +286,10 @@ def ring_flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, causal=Fals
     """q,k,v: [B, S_local, H, D] (rank r of `group` holds sequence chunk r).
     Returns out, or (out, lse [B,Hq,S_local] fp32, None) with return_attn_probs.
     Counterpart of sp_aurora/intel_ring_flash_attn.py:399."""
+    check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
+    res = native.attention(q, k, v, softmax_scale, causal, deterministic, group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return RingFlashAttnFunc.apply(q, k, v, dropout_p, softmax_scale, causal, window_size,
                                    alibi_slopes, deterministic, return_attn_probs, group)
 
@@ -297,6 +301,10 @@ def ring_flash_attn_kvpacked_func(q, kv, dropout_p=0.0, softmax_scale=None, caus
     sp_aurora/intel_ring_flash_attn.py:371."""
     if kv.dim() != 5 or kv.shape[2] != 2:
         raise ValueError(f"kv must be [B, S, 2, H, D], got {tuple(kv.shape)}")
+    check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
+    res = native.attention_kvpacked(q, kv, softmax_scale, causal, deterministic, group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return RingFlashAttnFunc.apply(q, kv[:, :, 0], kv[:, :, 1], dropout_p, softmax_scale, causal,
                                    window_size, alibi_slopes, deterministic, return_attn_probs,
                                    group)
@@ -309,6 +317,10 @@ def ring_flash_attn_qkvpacked_func(qkv, dropout_p=0.0, softmax_scale=None, causa
     sp_aurora/intel_ring_flash_attn.py:344."""
     if qkv.dim() != 5 or qkv.shape[2] != 3:
         raise ValueError(f"qkv must be [B, S, 3, H, D], got {tuple(qkv.shape)}")
+    check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
+    res = native.attention_qkvpacked(qkv, softmax_scale, causal, deterministic, group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return RingFlashAttnFunc.apply(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], dropout_p,
                                    softmax_scale, causal, window_size, alibi_slopes, deterministic,
                                    return_attn_probs, group)

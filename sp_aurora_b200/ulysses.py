@@ -17,7 +17,7 @@ from typing import Optional
 import torch
 import torch.distributed as dist
 
-from . import _lib, local_attn
+from . import _lib, local_attn, native
 from .all_to_all import (SeqAllToAll4D, all_to_all_4D, heads_all_to_all_packed, reshard_lse,
                          seq_all_to_all_packed)
 from .local_attn import check_unsupported_kwargs
@@ -99,6 +99,10 @@ def ulysses_flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, causal=F
                             window_size=(-1, -1), alibi_slopes=None, deterministic=False,
                             return_attn_probs=False, group=None):
     """q,k,v: [B, S_local, H, D]. Counterpart of sp_aurora/intel_ulysses_attn.py:501."""
+    check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
+    res = native.attention(q, k, v, softmax_scale, causal, group=group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return UlyssesFlashAttnFunc.apply(q, k, v, dropout_p, softmax_scale, causal, window_size,
                                       alibi_slopes, deterministic, return_attn_probs, group)
 
@@ -109,6 +113,10 @@ def ulysses_flash_attn_kvpacked_func(q, kv, dropout_p=0.0, softmax_scale=None, c
     """kv: [B, S_local, 2, Hkv, D]. Counterpart of sp_aurora/intel_ulysses_attn.py:587."""
     if kv.dim() != 5 or kv.shape[2] != 2:
         raise ValueError(f"kv must be [B, S, 2, H, D], got {tuple(kv.shape)}")
+    check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
+    res = native.attention_kvpacked(q, kv, softmax_scale, causal, group=group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return UlyssesFlashAttnFunc.apply(q, kv[:, :, 0], kv[:, :, 1], dropout_p, softmax_scale,
                                       causal, window_size, alibi_slopes, deterministic,
                                       return_attn_probs, group)
@@ -120,6 +128,10 @@ def ulysses_flash_attn_qkvpacked_func(qkv, dropout_p=0.0, softmax_scale=None, ca
     """qkv: [B, S_local, 3, H, D]. Counterpart of sp_aurora/intel_ulysses_attn.py:549."""
     if qkv.dim() != 5 or qkv.shape[2] != 3:
         raise ValueError(f"qkv must be [B, S, 3, H, D], got {tuple(qkv.shape)}")
+    check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
+    res = native.attention_qkvpacked(qkv, softmax_scale, causal, group=group)
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return UlyssesFlashAttnFunc.apply(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], dropout_p,
                                       softmax_scale, causal, window_size, alibi_slopes,
                                       deterministic, return_attn_probs, group)
@@ -161,7 +173,8 @@ def select_flash_attn_impl(attn_type: "AttnType" = AttnType.FA):
     def attn_fn(q, k, v, dropout_p=0.0, softmax_scale=None, causal=False, window_size=(-1, -1),
                 softcap=0.0, alibi_slopes=None, deterministic=False, return_attn_probs=False):
         check_unsupported_kwargs(dropout_p, window_size, alibi_slopes, softcap)
-        out, lse = local_attn.LocalFlashAttnFunc.apply(q, k, v, softmax_scale, causal)
+        res = native.attention_local(q, k, v, softmax_scale, causal)
+        out, lse = res if res is not None else local_attn.LocalFlashAttnFunc.apply(q, k, v, softmax_scale, causal)
         return (out, lse) if return_attn_probs else out
 
     return attn_fn

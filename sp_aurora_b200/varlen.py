@@ -22,7 +22,7 @@ from typing import List, Optional
 import torch
 import torch.distributed as dist
 
-from . import _lib, local_attn, zigzag
+from . import _lib, local_attn, native, zigzag
 from .local_attn import check_unsupported_kwargs
 from .ring import RingFlashAttnFunc
 
@@ -72,9 +72,12 @@ class VarlenFlashAttnFunc(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None
 
 
-def _packed_one_rank(q, k, v, bq, bk, softmax_scale, causal, deterministic, return_attn_probs):
+def _packed_one_rank(q, k, v, bq, bk, softmax_scale, causal, deterministic, return_attn_probs, group):
     seqs = [(a, b - a, c, d - c, 0) for a, b, c, d in zip(bq, bq[1:], bk, bk[1:]) if b > a]
-    out, lse = VarlenFlashAttnFunc.apply(q, k, v, seqs, softmax_scale, causal, deterministic)
+    res = native.attention_packed(q, k, v, seqs, softmax_scale, causal, deterministic, group)
+    if res is None:
+        res = VarlenFlashAttnFunc.apply(q, k, v, seqs, softmax_scale, causal, deterministic)
+    out, lse = res
     return (out, lse, None) if return_attn_probs else out
 
 
@@ -92,7 +95,7 @@ def ring_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k=None, max_se
     if len(bq) != len(bk):
         raise ValueError("cu_seqlens_q and cu_seqlens_k describe different numbers of sequences")
     if bq[-1] > 0 and _one_rank(group):
-        return _packed_one_rank(q, k, v, bq, bk, softmax_scale, causal, deterministic, return_attn_probs)
+        return _packed_one_rank(q, k, v, bq, bk, softmax_scale, causal, deterministic, return_attn_probs, group)
     outs, lses = [], []
     for i in range(len(bq) - 1):
         qi, ki, vi = q[bq[i]:bq[i + 1]], k[bk[i]:bk[i + 1]], v[bk[i]:bk[i + 1]]
@@ -155,6 +158,9 @@ def zigzag_ring_flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, caus
     check_unsupported_kwargs(dropout_p, window_size, alibi_slopes)
     if not causal:
         raise ValueError("the zigzag layout is defined for causal attention")
+    res = native.attention(q, k, v, softmax_scale, True, deterministic, group)   # one rank: the plain order
+    if res is not None:
+        return (*res, None) if return_attn_probs else res[0]
     return ZigzagRingFlashAttnFunc.apply(q, k, v, softmax_scale, deterministic, return_attn_probs, group)
 
 
@@ -173,7 +179,7 @@ def zigzag_ring_flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k=None,
     if bq != bk:
         raise ValueError("the zigzag layout needs equal query and key lengths per sequence")
     if bq[-1] > 0 and _one_rank(group):
-        return _packed_one_rank(q, k, v, bq, bk, softmax_scale, True, deterministic, return_attn_probs)
+        return _packed_one_rank(q, k, v, bq, bk, softmax_scale, True, deterministic, return_attn_probs, group)
     outs, lses = [], []
     for i in range(len(bq) - 1):
         if bq[i + 1] == bq[i]:
