@@ -37,6 +37,7 @@ struct Api {
   decltype(&spa_attn_varlen_fwd) varlen_fwd;
   decltype(&spa_attn_varlen_bwd) varlen_bwd;
   decltype(&spa_bwd_delta) delta;
+  decltype(&spa_rope_rows) rope_rows;
   decltype(&spa_check_status) check_status;
   decltype(&spa_last_error) last_error;
 } api;
@@ -276,6 +277,52 @@ struct QkvPackedAttn : torch::autograd::Function<QkvPackedAttn> {
   }
 };
 
+// dst = rotated src, both [B,S,H,D] with a contiguous last dimension; dst may be src.
+void rope(const Tensor& src, const Tensor& dst, const Tensor& cos, const Tensor& sin, bool inverse) {
+  const int64_t n[4] = {1, src.size(0), src.size(1), src.size(2)};
+  const int64_t ss[4] = {0, src.stride(0), src.stride(1), src.stride(2)};
+  const int64_t ds[4] = {0, dst.stride(0), dst.stride(1), dst.stride(2)};
+  check(api.rope_rows(src.data_ptr(), dst.data_ptr(), n, ss, ds, src.size(3), dtype_code(src.scalar_type()),
+                      cos.data_ptr<float>(), sin.data_ptr<float>(), cos.size(0), 2, 0, inverse,
+                      at::cuda::getCurrentCUDAStream(src.device().index()).stream()),
+        "spa_rope_rows");
+}
+
+// A projection's output x [B,S,Hq+2*Hkv,D] whose head slices are q, k and v, q and k rotated first
+// when cos / sin are given. The kernels write the three gradients into the slices of one dx and
+// the rotation is undone there in place: slice by slice, autograd would fill a zero tensor per
+// slice, copy the slice in and add the tensors up (B=1, S=8192, 32/8 heads, D=128, rotated:
+// 4360 -> 4030 us with both projections).
+struct HeadsPackedAttn : torch::autograd::Function<HeadsPackedAttn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Options& o, int64_t hq, int64_t hkv,
+                               const std::optional<Tensor>& cos, const std::optional<Tensor>& sin) {
+    Tensor q = x.narrow(2, 0, hq), k = x.narrow(2, hq, hkv), v = x.narrow(2, hq + hkv, hkv);
+    ctx->saved_data["hq"] = hq;
+    ctx->saved_data["hkv"] = hkv;
+    if (!cos) return finish_forward(ctx, {x}, run_forward(q, k, v, o), o, false);
+    Tensor qk = at::empty({x.size(0), x.size(1), hq + hkv, x.size(3)}, x.options());
+    rope(x.narrow(2, 0, hq + hkv), qk, *cos, *sin, false);
+    return finish_forward(ctx, {x, qk, *cos, *sin},
+                          run_forward(qk.narrow(2, 0, hq), qk.narrow(2, hq, hkv), v, o), o, false);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Options o = load_options(ctx);
+    const int64_t hq = ctx->saved_data["hq"].toInt(), hkv = ctx->saved_data["hkv"].toInt();
+    const bool rotated = s.size() == 6;
+    const Tensor &x = s[0], &qk = rotated ? s[1] : s[0], &out = s[s.size() - 2], &lse = s[s.size() - 1];
+    Tensor dx = at::empty(x.sizes(), x.options());
+    run_backward(grad_or_zeros(grads, out), qk.narrow(2, 0, hq), qk.narrow(2, hq, hkv), x.narrow(2, hq + hkv, hkv), out,
+                 lse, dx.narrow(2, 0, hq), dx.narrow(2, hq, hkv), dx.narrow(2, hq + hkv, hkv), o);
+    if (rotated) {
+      const Tensor dqk = dx.narrow(2, 0, hq + hkv);
+      rope(dqk, dqk, s[2], s[3], true);
+    }
+    end_of_backward();
+    return {dx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
 using Result = std::optional<std::tuple<Tensor, Tensor>>;
 
 // Runs f without the interpreter lock, with the tensors' device current.
@@ -323,6 +370,21 @@ Result attention_qkvpacked(const Tensor& x, std::optional<double> scale, bool ca
   return released(x, [&] { return QkvPackedAttn::apply(x, o); });
 }
 
+Result attention_heads_packed(const Tensor& x, int64_t hq, int64_t hkv, const std::optional<Tensor>& cos,
+                              const std::optional<Tensor>& sin, bool causal) {
+  if (!quiet_context() || !plain(x) || x.dim() != 4 || x.stride(3) != 1 || x.numel() == 0 || hkv <= 0 || hq % hkv ||
+      x.size(2) != hq + 2 * hkv || dtype_code(x.scalar_type()) < 0 || !takes_head_dim(x.size(3)) ||
+      cos.has_value() != sin.has_value())
+    return std::nullopt;
+  for (const auto* t : {&cos, &sin})
+    if (t->has_value() && (!plain(**t) || (*t)->scalar_type() != at::kFloat || (*t)->dim() != 2 ||
+                           (*t)->size(1) != x.size(3) / 2 || !(*t)->is_contiguous() || (*t)->requires_grad() ||
+                           (*t)->device() != x.device()))
+      return std::nullopt;
+  const Options o = options(std::nullopt, x.size(3), causal, false);
+  return released(x, [&] { return HeadsPackedAttn::apply(x, o, hq, hkv, cos, sin); });
+}
+
 Result attention_packed(const Tensor& q, const Tensor& k, const Tensor& v,
                         const std::vector<std::tuple<int, int, int, int, int>>& seqs, std::optional<double> scale,
                         bool causal, bool deterministic) {
@@ -334,7 +396,7 @@ Result attention_packed(const Tensor& q, const Tensor& k, const Tensor& v,
 }
 
 void set_api(const std::vector<uintptr_t>& f, pybind11::object error) {
-  TORCH_CHECK(f.size() == 9, "nine entry points expected");
+  TORCH_CHECK(f.size() == 10, "ten entry points expected");
   api.fwd = reinterpret_cast<decltype(api.fwd)>(f[0]);
   api.fwd_workspace = reinterpret_cast<decltype(api.fwd_workspace)>(f[1]);
   api.fwd_ws = reinterpret_cast<decltype(api.fwd_ws)>(f[2]);
@@ -344,6 +406,7 @@ void set_api(const std::vector<uintptr_t>& f, pybind11::object error) {
   api.delta = reinterpret_cast<decltype(api.delta)>(f[6]);
   api.check_status = reinterpret_cast<decltype(api.check_status)>(f[7]);
   api.last_error = reinterpret_cast<decltype(api.last_error)>(f[8]);
+  api.rope_rows = reinterpret_cast<decltype(api.rope_rows)>(f[9]);
   spa_error = error.release().ptr();
 }
 
@@ -355,4 +418,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention_kvpacked", &attention_kvpacked);
   m.def("attention_qkvpacked", &attention_qkvpacked);
   m.def("attention_packed", &attention_packed);
+  m.def("attention_heads_packed", &attention_heads_packed);
 }

@@ -19,7 +19,7 @@ except ImportError as e:
 
 _native.set_api([C.cast(getattr(_lib.lib, name), C.c_void_p).value for name in (
     "spa_attn_fwd", "spa_attn_fwd_workspace", "spa_attn_fwd_ws", "spa_attn_bwd", "spa_attn_varlen_fwd",
-    "spa_attn_varlen_bwd", "spa_bwd_delta", "spa_check_status", "spa_last_error")], _lib.SpaError)
+    "spa_attn_varlen_bwd", "spa_bwd_delta", "spa_check_status", "spa_last_error", "spa_rope_rows")], _lib.SpaError)
 
 
 def _general(group) -> bool:
@@ -57,6 +57,15 @@ def attention_qkvpacked(qkv, softmax_scale, causal, deterministic=False, group=N
     if _general(group):
         return None
     return _native.attention_qkvpacked(qkv, _scale(softmax_scale), bool(causal), bool(deterministic))
+
+
+def attention_heads_packed(x, hq, hkv, cos, sin, causal, group=None):
+    """x [B,S,hq+2*hkv,D]: q, k and v side by side, as one projection writes them; with cos and
+    sin (see rope_tables) q and k are rotated, positions from 0. The gradient is written in
+    that layout."""
+    if _general(group):
+        return None
+    return _native.attention_heads_packed(x, hq, hkv, cos, sin, bool(causal))
 
 
 def attention_packed(q, k, v, seqs, softmax_scale, causal, deterministic=False, group=None):

@@ -145,3 +145,25 @@ def test_forward_and_backward_are_captured_in_a_graph():
     torch.cuda.synchronize()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["ring", "ulysses"])
+@pytest.mark.parametrize("rope_base", [None, 10000.0])
+def test_block_node_equals_the_sliced_form(general, mode, rope_base):
+    """Rotation, attention and the joined gradient of one projection output. Bitwise: adding the
+    zeros of the other slices changes nothing, the rotation is undone from the same 16-bit rows."""
+    import sp_aurora_b200 as spa
+    torch.manual_seed(4)
+    blk = spa.SequenceParallelAttentionBlock(512, 4, 2, mode=mode, device="cuda", rope_base=rope_base)
+    x, dy = _randn(2, 129, 512), _randn(2, 129, 512)
+
+    def step():
+        t = x.clone().requires_grad_(True)
+        y = blk(t, causal=True)
+        return [y.detach(), *torch.autograd.grad(y, (t, *blk.parameters()), dy)]
+    a = step()
+    with general():
+        b = step()
+    spa.check_status()
+    for p, q in zip(a, b):
+        assert torch.equal(p, q)
