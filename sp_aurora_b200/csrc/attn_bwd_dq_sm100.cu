@@ -497,6 +497,7 @@ int launch_dq_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
     set_error("q base and strides must be 16-byte aligned");
     return SPA_EINVAL;
   }
+  if (dq_loops(a, seqs, n_seq)) return launch_bwd_dq_loop_sm100(a, seqs, n_seq);
   if (a->D == 128) {
     return bf ? launch_dq_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
               : launch_dq_typed<128, __half, kVar>(a, 0, seqs, n_seq);

@@ -50,6 +50,10 @@ int launch_bwd_dkv_sm100(const spa_bwd_args* a);      // K/V-stationary pass: dK
 int launch_fwd_sm100_var(const spa_fwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_bwd_dq_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
+// The dQ pass with CTAs that loop over query tiles, and the rule that takes a launch there
+// (n_seq = 0: a plain one).
+bool dq_loops(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
+int launch_bwd_dq_loop_sm100(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_fwd_simt(const spa_fwd_args* a);
 int launch_bwd_simt(const spa_bwd_args* a);
 
