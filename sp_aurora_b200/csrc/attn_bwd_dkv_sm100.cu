@@ -344,8 +344,9 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       const int hq = g * G + it / n_q;
       const int qi = (i_start + it % n_q) * kTileQ + (stat_tid & 127);
       const size_t idx = (size_t)b * p.lse_sb + (size_t)hq * p.lse_sh + q_row0 + qi;
-      if (stat_tid < 128) return qi < Sq ? -p.lse[idx] * kLog2e : -INFINITY;
-      return qi < Sq ? -p.delta[idx] : 0.f;
+      // past the L1, which a start beside the dQ pass need not invalidate
+      if (stat_tid < 128) return qi < Sq ? -__ldcg(p.lse + idx) * kLog2e : -INFINITY;
+      return qi < Sq ? -__ldcg(p.delta + idx) : 0.f;
     };
     if (n_it > 0 && stat_tid < 256) {
       row_buf[(0 * 2 + (stat_tid >> 7)) * kTileQ + (stat_tid & 127)] = fetch_rowstat(0);
@@ -557,6 +558,7 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  grid_acquire();   // launched beside the dQ pass: this grid must not end before that one
 }
 
 // One CTA per (K/V tile, kv head, batch) leaves the last wave partly empty when that count
@@ -592,7 +594,7 @@ int choose_q_split(const spa_bwd_args* a, long long base_grid) {
 }
 
 template <int D, typename T, bool kVar>
-int launch_dkv_typed(const spa_bwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq) {
+int launch_dkv_typed(const spa_bwd_args* a, int is_bf16, const spa_seq* seqs, int n_seq, bool behind_dq) {
   using L = DkvSmem<D>;
   CUtensorMap tq, tk, tv, tdo, tdk, tdv;
   if (encode_rows_map(&tq, a->q, is_bf16, D, a->Sq, a->Hq, a->B, a->q_ss, a->q_sh, a->q_sb, kTileQ))
@@ -652,9 +654,20 @@ int launch_dkv_typed(const spa_bwd_args* a, int is_bf16, const spa_seq* seqs, in
       set_error("bwd dkv memset: %s", cudaGetErrorString(e));
       return SPA_ECUDA;
     }
+    behind_dq = false;
   }
-  kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, tdo, tdk, tdv, p, var);
-  cudaError_t e = cudaGetLastError();
+  // Beside the dQ pass where its walks are long enough for the overlap to show: 4096 causal rows
+  // of 4 heads (64 CTAs here, 128 there) delta + dQ + dK/dV 200 -> 139 us, 2048 rows of 8 heads
+  // 67 -> 44, 2 x 3001 rows of 32 550 -> 538. Below 12 tiles a call waits for the host, and the
+  // attribute costs it 1 us.
+  int longest = a->Sk;
+  for (int i = 0; i < n_seq; ++i) longest = i ? std::max(longest, seqs[i].sk) : seqs[i].sk;
+  cudaError_t e = cudaSuccess;
+  if (behind_dq && ceil_div(longest, kTileKV) >= 12)
+    e = launch_programmatic(kern, grid, kThreads, smem_bytes, a->stream, tq, tk, tv, tdo, tdk, tdv, p, var);
+  else
+    kern<<<(unsigned)grid, kThreads, smem_bytes, (cudaStream_t)a->stream>>>(tq, tk, tv, tdo, tdk, tdv, p, var);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("bwd dkv sm100 launch: %s", cudaGetErrorString(e));
     return SPA_ECUDA;
@@ -663,7 +676,7 @@ int launch_dkv_typed(const spa_bwd_args* a, int is_bf16, const spa_seq* seqs, in
 }
 
 template <bool kVar>
-int launch_dkv_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
+int launch_dkv_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq, bool behind_dq) {
   const bool bf = a->dtype == SPA_DTYPE_BF16;
   if (!a->dkv_fp32 &&
       (((uintptr_t)a->dk & 15) || ((uintptr_t)a->dv & 15) || ((a->dkv_ss * 2) & 15) ||
@@ -672,11 +685,11 @@ int launch_dkv_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
     return SPA_EINVAL;
   }
   if (a->D == 128) {
-    return bf ? launch_dkv_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
-              : launch_dkv_typed<128, __half, kVar>(a, 0, seqs, n_seq);
+    return bf ? launch_dkv_typed<128, __nv_bfloat16, kVar>(a, 1, seqs, n_seq, behind_dq)
+              : launch_dkv_typed<128, __half, kVar>(a, 0, seqs, n_seq, behind_dq);
   } else if (a->D == 64) {
-    return bf ? launch_dkv_typed<64, __nv_bfloat16, kVar>(a, 1, seqs, n_seq)
-              : launch_dkv_typed<64, __half, kVar>(a, 0, seqs, n_seq);
+    return bf ? launch_dkv_typed<64, __nv_bfloat16, kVar>(a, 1, seqs, n_seq, behind_dq)
+              : launch_dkv_typed<64, __half, kVar>(a, 0, seqs, n_seq, behind_dq);
   }
   set_error("tensor-core backward supports head_dim 64 and 128, got %d", a->D);
   return SPA_EUNSUPPORTED;
@@ -684,10 +697,12 @@ int launch_dkv_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
 
 }  // namespace
 
-int launch_bwd_dkv_sm100(const spa_bwd_args* a) { return launch_dkv_any<false>(a, nullptr, 0); }
+int launch_bwd_dkv_sm100(const spa_bwd_args* a, bool behind_dq) {
+  return launch_dkv_any<false>(a, nullptr, 0, behind_dq);
+}
 
-int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
-  return launch_dkv_any<true>(a, seqs, n_seq);
+int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq, bool behind_dq) {
+  return launch_dkv_any<true>(a, seqs, n_seq, behind_dq);
 }
 
 }  // namespace spa

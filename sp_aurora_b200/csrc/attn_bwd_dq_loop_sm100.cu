@@ -173,6 +173,7 @@ attn_bwd_dq_loop_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wc{p.status, cta_abort};
+  grid_release();   // as in attn_bwd_dq_sm100.cu
 
   if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA

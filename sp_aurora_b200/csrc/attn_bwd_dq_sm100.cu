@@ -177,6 +177,9 @@ attn_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tm_k,
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wc{p.status, cta_abort};
+  // The dK/dV pass may start once every CTA of this grid is running: it reads nothing that this
+  // grid writes, and what both read was complete before this grid started.
+  grid_release();
 
   if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA

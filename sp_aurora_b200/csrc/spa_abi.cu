@@ -929,7 +929,7 @@ static int run_bwd(const spa_bwd_args* a) {
   int rc = SPA_OK;
   if (tensor_core) {
     if (want_dq) rc = launch_bwd_dq_sm100(a);
-    if (rc == SPA_OK && want_dkv) rc = launch_bwd_dkv_sm100(a);
+    if (rc == SPA_OK && want_dkv) rc = launch_bwd_dkv_sm100(a, want_dq);
   } else {
     rc = launch_bwd_simt(a);
   }
@@ -971,7 +971,7 @@ int spa_attn_varlen_bwd(const spa_bwd_args* args, const spa_seq* seqs, int32_t n
     for (int i = 0; i < n_seq && rc == SPA_OK; i += kVarMaxSeqs) {
       const int m = std::min(kVarMaxSeqs, n_seq - i);
       rc = launch_bwd_dq_sm100_var(&n, seqs + i, m);
-      if (rc == SPA_OK) rc = launch_bwd_dkv_sm100_var(&n, seqs + i, m);
+      if (rc == SPA_OK) rc = launch_bwd_dkv_sm100_var(&n, seqs + i, m, true);
       if (rc == SPA_OK) note_launch(2);
     }
     return rc;

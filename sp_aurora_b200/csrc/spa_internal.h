@@ -45,17 +45,37 @@ int device_sm_count();
 int64_t fwd_sm100_workspace(const spa_fwd_args* a);
 int launch_fwd_sm100(const spa_fwd_args* a, float* workspace);
 int launch_bwd_dq_sm100(const spa_bwd_args* a);       // query-stationary pass: dQ
-int launch_bwd_dkv_sm100(const spa_bwd_args* a);      // K/V-stationary pass: dK, dV
+// K/V-stationary pass: dK, dV. behind_dq: the dQ pass of the same problem is the kernel just
+// before it in the stream; the two may then overlap where one drains and the other fills.
+int launch_bwd_dkv_sm100(const spa_bwd_args* a, bool behind_dq);
 // The same kernels over up to kVarMaxSeqs sequences of a packed batch (B = 1).
 int launch_fwd_sm100_var(const spa_fwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_bwd_dq_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
-int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
+int launch_bwd_dkv_sm100_var(const spa_bwd_args* a, const spa_seq* seqs, int n_seq, bool behind_dq);
 // The dQ pass with CTAs that loop over query tiles, and the rule that takes a launch there
 // (n_seq = 0: a plain one).
 bool dq_loops(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_bwd_dq_loop_sm100(const spa_bwd_args* a, const spa_seq* seqs, int n_seq);
 int launch_fwd_simt(const spa_fwd_args* a);
 int launch_bwd_simt(const spa_bwd_args* a);
+
+// kern<<<grid, threads, smem, stream>>>(args...), with the programmatic attribute: the grid may
+// start before the one in front of it has ended (see grid_release / grid_acquire).
+template <typename... P, typename... A>
+cudaError_t launch_programmatic(void (*kern)(P...), long long grid, int threads, int smem, void* stream,
+                                const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 

@@ -61,6 +61,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Programmatic dependent launch. grid_release: the next kernel of the stream, if it was launched
+// with the programmatic attribute, may start as soon as every CTA of this grid has got here.
+// grid_acquire: wait until the grid before this one has completed and its writes are visible
+// (returns at once in a kernel launched without the attribute).
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_acquire() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Hand registers from one warpgroup to another (every warp of the warpgroup must get here). What
 // the growing warpgroups take has to be given up by the others: the block owns what it was
 // launched with.
