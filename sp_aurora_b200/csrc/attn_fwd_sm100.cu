@@ -54,6 +54,7 @@ struct FwdParams {
   int n_qblk;
   int chunk;   // query blocks per scheduling chunk (n_qblk or 1)
   int row_step, head_step;   // tile 1 of a CTA = tile 0 + so many query rows and heads
+  int one_tile;              // the CTA has no tile 1 (row_step = head_step = 0)
   int split;   // CTAs sharing the keys of a block; > 1: partial results go to `part`
   float* part;               // [split][B][Sq][Hq][D] normalised outputs, then [split][B][Hq][Sq] lse
   float scale_log2;
@@ -129,7 +130,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   // S=131072 causal 993 -> 1036 TFLOP/s), or one block for small causal problems, where
   // longest-block-first over all heads matters more. Packed sequences: heads fastest, then
   // the blocks of all sequences by falling distance from the start of their sequence.
-  const int row_step = kMode == kCut ? p.row_step : kTileM;
+  const int row_step = kMode == kPlain ? kTileM : p.row_step;
+  const bool one_tile = kMode != kPlain && p.one_tile;
   const int head_step = kMode == kCut ? p.head_step : 0;
   int w = blockIdx.x;
   int h, b, qblk, sg = 0, ks = 0;
@@ -165,7 +167,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
   for (int t = 0; t < 2; ++t) {
     const int r0 = q0 + t * row_step;
     int n = 0;
-    if (r0 < Sq) {
+    if (r0 < Sq && !(one_tile && t == 1)) {
       n = (Sk + kTileN - 1) / kTileN;
       if (p.causal) {
         const int last_row = min(r0 + kTileM, Sq) - 1;
@@ -220,7 +222,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(v_map);
-      const int q_tiles = (n_t[1] > 0 || q0 + row_step < Sq) ? 2 : 1;
+      const int q_tiles = !one_tile && (n_t[1] > 0 || q0 + row_step < Sq) ? 2 : 1;
       mbar_arrive_expect_tx(q_full, q_tiles * L::kTileBytes);
       for (int t = 0; t < q_tiles; ++t)
         for (int s = 0; s < D / 64; ++s)
@@ -416,7 +418,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
       ok = warp_wait(&o_done[t], (nt - 1) & 1, wc, 12 + t, nt);
       tc_fence_after();
     }
-    if (ok) {
+    if (ok && !(one_tile && t == 1)) {
       const bool row_ok = qrow < Sq;
       const bool have = (nt > 0) && (l > 0.f);
       const float inv_l = have ? 1.f / l : 0.f;
@@ -546,6 +548,7 @@ combine_splits_kernel(const FwdParams p) {
 
 struct FwdPlan {
   bool pair_heads;   // the two tiles of a CTA are one query tile of two heads of a kv group
+  bool one_tile;     // a CTA has one query tile only
   int split;
 };
 
@@ -555,35 +558,44 @@ struct FwdPlan {
 // chip, or one causal block outlasts everything else, the keys of each block are cut into
 // `split` slices whose partial results a second kernel joins. `workspace` false: no splitting.
 // 128 queries of 32 / 8 heads over 16384 keys, batch 2, D=128: 250 -> 95 us; 40 queries of 8 heads over 8000 keys: 119 -> 28; 4096 causal rows of 4 heads: 76 -> 54.
-// Times are in units of one key tile of both query tiles (2.2 us).
+// A grid that fills less than half of the chip takes one query tile per CTA: alone, a tile goes
+// through a key tile in 0.7 of the time that two need in turn, and there are SMs to spare.
+// Times are in units of one key tile of two query tiles (2.2 us).
 FwdPlan plan_fwd(const spa_fwd_args* a, bool workspace) {
-  FwdPlan plan{false, 1};
+  FwdPlan plan{false, false, 1};
   const int tiles = ceil_div(a->Sq, kTileM);
   plan.pair_heads = tiles % 2 == 1 && tiles <= 5 && (a->Hq / a->Hkv) % 2 == 0;
-  if (!workspace || a->merge_prev || a->out_acc) return plan;
-  const long long blocks = plan.pair_heads ? (long long)tiles * (a->Hq / 2) * a->B
-                                           : (long long)ceil_div(tiles, 2) * a->Hq * a->B;
+  const long long heads = (long long)a->Hq * a->B;
+  const long long pairs = plan.pair_heads ? tiles * heads / 2 : ceil_div(tiles, 2) * heads;
   const int n_sm = device_sm_count();
-  if (blocks >= 2ll * n_sm) return plan;
+  if (pairs >= 2ll * n_sm) return plan;
+  const bool may_split = workspace && !a->merge_prev && !a->out_acc;
   long long longest = ceil_div(a->Sk, kTileN);
   if (a->causal)
     longest = std::max(0ll, std::min(longest, ((long long)a->Sq - 1 + a->causal_off) / kTileN + 1));
   const double mean = a->causal && a->causal_off < a->Sk ? 0.5 * (longest + 1) : (double)longest;
   const double fill = 1.5;             // prologue and epilogue of a CTA
-  const double rows = (double)a->B * a->Sq * a->Hq;
-  double best = 0.0;
-  for (int s = 1; s <= 16; ++s) {
-    if (s > 1 && longest / s < 4) break;
-    const double waves = (double)((blocks * s + n_sm - 1) / n_sm);
-    const double work = blocks * s * (mean / s + fill) / n_sm;
-    const double step = longest / (double)s + fill;
-    double t = a->causal ? std::max(step, work) : waves * step;
-    if (s > 1) t += 2.5 + s * rows * a->D * 8.0 / 1e7;   // join: a launch, and its bytes through L2
-    if (s == 1 || t < best * 0.93) {
-      best = t;
-      plan.split = s;
+  const double rows = (double)heads * a->Sq;
+  double best = -1.0;
+  for (int one = 0; one < 2; ++one) {
+    const long long blocks = one ? tiles * heads : pairs;
+    if (one && blocks > n_sm) break;
+    const double unit = one ? 0.7 : 1.0;
+    for (int s = 1; s <= (may_split ? 16 : 1); ++s) {
+      if (s > 1 && longest / s < 4) break;
+      const double waves = (double)((blocks * s + n_sm - 1) / n_sm);
+      const double work = blocks * s * (unit * mean / s + fill) / n_sm;
+      const double step = unit * longest / s + fill;
+      double t = a->causal ? std::max(step, work) : waves * step;
+      if (s > 1) t += 2.5 + s * rows * a->D * 8.0 / 1e7;   // join: a launch, and its bytes through L2
+      if (best < 0.0 || t < best * 0.93) {
+        best = t;
+        plan.one_tile = one;
+        plan.split = s;
+      }
     }
   }
+  if (plan.one_tile) plan.pair_heads = false;
   return plan;
 }
 
@@ -602,7 +614,8 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, in
   FwdParams p;
   p.B = a->B; p.Sq = a->Sq; p.Sk = a->Sk; p.Hq = a->Hq; p.Hkv = a->Hkv;
   p.causal = a->causal; p.causal_off = a->causal_off; p.merge_prev = a->merge_prev;
-  p.row_step = plan.pair_heads ? 0 : kTileM;
+  p.one_tile = plan.one_tile;
+  p.row_step = plan.pair_heads || plan.one_tile ? 0 : kTileM;
   p.head_step = plan.pair_heads ? 1 : 0;
   p.split = plan.split;
   p.part = part;
@@ -620,7 +633,7 @@ int launch_fwd_typed(const spa_fwd_args* a, int is_bf16, const spa_seq* seqs, in
   long long grid = (long long)p.n_qblk * a->B * (a->Hq >> p.head_step) * p.split;
   VarTable<kVar, 1> var;
   if constexpr (kVar) {
-    grid = fill_var_table(&var, seqs, n_seq, 2 * kTileM, /*by_key=*/false) * a->Hq;
+    grid = fill_var_table(&var, seqs, n_seq, kTileM + p.row_step, /*by_key=*/false) * a->Hq;
     for (int i = 0; i < n_seq; ++i) {
       const VarSeq& q = var.s[i];
       if (encode_rows_map(&var.tm[i][0], row_ptr(a->v, q.k0, a->v_ss), is_bf16, D, q.sk, a->Hkv, 1, a->v_ss,
@@ -668,12 +681,14 @@ int64_t fwd_sm100_workspace(const spa_fwd_args* a) {
 
 int launch_fwd_sm100(const spa_fwd_args* a, float* workspace) {
   const FwdPlan plan = plan_fwd(a, workspace != nullptr);
-  return plan.pair_heads || plan.split > 1 ? launch_fwd_any<kCut>(a, nullptr, 0, plan, workspace)
+  return plan.pair_heads || plan.one_tile || plan.split > 1 ? launch_fwd_any<kCut>(a, nullptr, 0, plan, workspace)
                                            : launch_fwd_any<kPlain>(a, nullptr, 0, plan, nullptr);
 }
 
 int launch_fwd_sm100_var(const spa_fwd_args* a, const spa_seq* seqs, int n_seq) {
-  return launch_fwd_any<kVarlen>(a, seqs, n_seq, FwdPlan{false, 1}, nullptr);
+  long long tiles = 0;   // one query tile per CTA while that fits the chip, as in plan_fwd
+  for (int i = 0; i < n_seq; ++i) tiles += ceil_div(seqs[i].sq, kTileM);
+  return launch_fwd_any<kVarlen>(a, seqs, n_seq, FwdPlan{false, tiles * a->Hq <= device_sm_count(), 1}, nullptr);
 }
 
 }  // namespace spa
