@@ -95,9 +95,12 @@ def _segments(cu_q, cu_k) -> List[Tuple[int, int, int, int]]:
     return segs
 
 
-def _one_launch(segs, Tq: int, Tk: int) -> bool:
-    """Segments the packed kernels take as they are: rising, inside the tensors. (Tables made by
-    llama3_flash_attn_prepare_cu_seqlens always are.)"""
+def _one_launch(segs, Tq: int, k, k_slice) -> bool:
+    """Segments the packed kernels take as they are: rising, inside the tensors, over a view of the
+    keys. (Tables made by llama3_flash_attn_prepare_cu_seqlens always are.)"""
+    if not isinstance(k_slice, slice):
+        return False
+    Tk = k[k_slice].shape[0]
     ends = [0, 0]
     for qa, qb, ka, kb in segs:
         if qa < ends[0] or ka < ends[1]:
@@ -155,7 +158,7 @@ def llama3_forward(group, q, k, v, segs, k_slice: slice, heads_k_stride: int, so
     g = Hq // Hkv
     out = torch.empty_like(q)
     lse = torch.empty((Hq, Tl), dtype=torch.float32, device=q.device)
-    if W == 1 and fwd_step is local_attn.attn_fwd_step and _one_launch(segs, Tl, k[k_slice].shape[0]):
+    if W == 1 and fwd_step is local_attn.attn_fwd_step and _one_launch(segs, Tl, k, k_slice):
         fwd_step(q.unsqueeze(0), k[k_slice].unsqueeze(0), v[k_slice].unsqueeze(0), softmax_scale, causal,
                  lse.unsqueeze(0), out=out.unsqueeze(0), seqs=_seqs(segs))
         return out, lse
@@ -186,7 +189,7 @@ def llama3_backward(group, dout, q, k, v, out, lse, segs, k_slice: slice, heads_
     Tl, Hq, D = q.shape
     Hkv = k.shape[1]
     g = Hq // Hkv
-    if W == 1 and bwd_step is local_attn.attn_bwd_step and _one_launch(segs, Tl, k[k_slice].shape[0]):
+    if W == 1 and bwd_step is local_attn.attn_bwd_step and _one_launch(segs, Tl, k, k_slice):
         return local_attn.packed_backward(dout, q, k, v, out, lse, _seqs(segs), softmax_scale, causal,
                                           deterministic, k_slice)
     dt = q.dtype
@@ -265,8 +268,10 @@ def _native_one_rank(q, k, v, cu_q, cu_k, heads_k_stride, k_slice, softmax_scale
             (heads_k_stride and (int(heads_k_stride) <= 0 or k.shape[1] % int(heads_k_stride))):
         return None
     segs = _segments(cu_q, cu_k)
-    start, stop, step = k_slice.indices(k.shape[0])
-    if step != 1 or not _one_launch(segs, q.shape[0], stop - start) or segs[-1][1] != q.shape[0]:
+    if not _one_launch(segs, q.shape[0], k, k_slice) or segs[-1][1] != q.shape[0]:
+        return None
+    start, _, step = k_slice.indices(k.shape[0])
+    if step != 1:
         return None
     seqs = [(q0, sq, start + k0, sk, off) for q0, sq, k0, sk, off in _seqs(segs)]
     return native.attention_packed(q, k, v, seqs, softmax_scale, causal, deterministic, group)

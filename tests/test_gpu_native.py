@@ -167,3 +167,29 @@ def test_block_node_equals_the_sliced_form(general, mode, rope_base):
     spa.check_status()
     for p, q in zip(a, b):
         assert torch.equal(p, q)
+
+
+def test_other_modes():
+    """inference_mode, create_graph, a dispatch mode and a non-default stream."""
+    import sp_aurora_b200 as spa
+    from torch.utils._python_dispatch import TorchDispatchMode
+    q, kv = _randn(1, 130, 4, 64), _randn(1, 130, 2, 2, 64)
+    want = spa.ring_flash_attn_kvpacked_func(q, kv, causal=True)
+    with torch.inference_mode():
+        assert torch.equal(spa.ring_flash_attn_kvpacked_func(q, kv, causal=True), want)
+
+    class Seen(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    with Seen():
+        assert torch.equal(spa.ring_flash_attn_kvpacked_func(q, kv, causal=True), want)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        x = q.clone().requires_grad_(True)
+        out = spa.ring_flash_attn_kvpacked_func(x, kv, causal=True)
+        g, = torch.autograd.grad(out, x, torch.ones_like(out), create_graph=True)
+    torch.cuda.current_stream().wait_stream(side)
+    y = q.clone().requires_grad_(True)
+    h, = torch.autograd.grad(spa.ring_flash_attn_kvpacked_func(y, kv, causal=True), y, torch.ones_like(want))
+    assert torch.equal(out, want) and torch.equal(g, h)
