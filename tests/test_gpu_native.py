@@ -120,9 +120,10 @@ def test_what_the_node_leaves_to_the_general_way():
         torch.autograd.grad(out, x, g)
 
 
-def test_forward_and_backward_are_captured_in_a_graph():
+@pytest.mark.parametrize("S", [500, 2000])     # 2000: the dK/dV pass starts beside the dQ pass, keys split
+def test_forward_and_backward_are_captured_in_a_graph(S):
     import sp_aurora_b200 as spa
-    q, k, v, do = (_randn(1, 500, 4, 128) for _ in range(4))
+    q, k, v, do = (_randn(1, S, 4, 128) for _ in range(4))
     leaves = [t.requires_grad_(True) for t in (q, k, v)]
 
     def step():
