@@ -13,8 +13,8 @@
 // the next product's operand go through shared memory rows that only their own warp reads (no
 // block barrier). Tile rows are padded by four floats, which puts the 16 rows a half-warp reads
 // at once in different banks. B=2, S=1024, 32 heads, D=64, causal, fp32: forward + backward
-// 2486 -> 1127 us against four threads per row with one float4 load per four multiply-adds;
-// the three kernels now run at 30, 36 and 36 TFLOP/s executed of the 73 an FMA-only loop reaches.
+// 2486 -> 1151 us against four threads per row with one float4 load per four multiply-adds;
+// the three kernels now run at 29, 35 and 35 TFLOP/s executed of the 73 an FMA-only loop reaches.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math.h>
@@ -104,20 +104,21 @@ __device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t stri
 }
 
 // acc[i][j] = row (ty + i*kTy) of a . row (tx + 16*j) of b. The even and the odd elements are
-// summed apart (the packed multiply-add works on pairs) and joined every 64 elements: a chain of
-// 64 terms per sum at D = 128 left the gradients 14 % further from 64-bit results.
+// summed apart (the packed multiply-add works on pairs) and joined every 32 elements. Joined at the
+// end only, results were up to 14 % (D = 128) and 4 % (D = 64) further from 64-bit ones than those of
+// four threads per row; joining costs 2 % of the time (1127 -> 1151 us for the call above).
 template <int D, int R>
 __device__ __forceinline__ void dot_tiles(float (&acc)[R][kCols], const float* a, const float* b, int ty, int tx) {
   using S = SimtShape<D, R>;
 #pragma unroll
-  for (int f0 = 0; f0 < D; f0 += 64) {
+  for (int f0 = 0; f0 < D; f0 += 32) {
     float2 p[R][kCols];
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int j = 0; j < kCols; ++j) p[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 2
-    for (int f = f0; f < (D < f0 + 64 ? D : f0 + 64); f += 4) {
+    for (int f = f0; f < f0 + 32; f += 4) {
       float4 bv[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) bv[j] = *reinterpret_cast<const float4*>(b + (tx + 16 * j) * S::kLd + f);
