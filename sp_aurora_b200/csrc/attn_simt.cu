@@ -302,10 +302,12 @@ attn_fwd_simt_kernel(const SimtFwdParams p) {
 #pragma unroll
       for (int c = 0; c < S::kNC; ++c) tile[i][c] = 0.f;
     add_product<D, R>(tile, p_s, v_s, ty, tx);
+    // A row that has seen no key yet keeps its zeros: its weights are 0, but 0 * Inf in V is not.
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
-      for (int c = 0; c < S::kNC; ++c) o[i][c] = fmaf(o[i][c], alpha[i], tile[i][c]);
+      for (int c = 0; c < S::kNC; ++c)
+        o[i][c] = m[i] == -INFINITY ? 0.f : fmaf(o[i][c], alpha[i], tile[i][c]);
   }
 
 #pragma unroll
@@ -319,7 +321,7 @@ attn_fwd_simt_kernel(const SimtFwdParams p) {
     lse_old = __shfl_sync(0xffffffffu, lse_old, threadIdx.x & 16);
     if (row >= p.Sq) continue;
     const bool have = l[i] > 0.f;
-    const float inv_l = have ? 1.f / l[i] : 0.f;
+    const float inv_l = have ? 1.f / l[i] : l[i];   // 0 without a key, NaN stays NaN
     const float lse_blk = have ? m[i] + logf(l[i]) : -INFINITY;
     float w_old = 0.f, w_blk = have ? 1.f : 0.f, lse_new = lse_blk;
     if (p.merge_prev) {

@@ -41,3 +41,30 @@ def test_fp32_tiles_match_the_oracle(Sq, Sk, D, causal, off):
     gk, gv = (t.view(B, Hkv, Hq // Hkv, Sk, D).sum(2) for t in (gk, gv))
     for got, want in ((out, o), (dq, gq), (dkv[:, :, 0], gk), (dkv[:, :, 1], gv)):
         assert (got.cpu().double().transpose(1, 2) - want).abs().max() <= 1e-5 * max(1.0, want.abs().max().item())
+
+
+def _forward(q, k, v, causal, off=0, scale=None, **kw):
+    from sp_aurora_b200 import local_attn as la
+    out = torch.empty_like(q)
+    lse = kw.pop("lse", None)
+    if lse is None:
+        lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], device="cuda")
+    la.attn_fwd_step(q, k, v, scale or q.shape[-1] ** -0.5, causal, lse, out=out, causal_off=off, **kw)
+    return out, lse
+
+
+@pytest.mark.parametrize("D,dtype", [(32, torch.bfloat16), (64, torch.float32), (128, torch.float32)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_rows_without_a_visible_key_ignore_the_values(D, dtype, bad):
+    """Query i sees the keys up to i - 10: rows 0-9 give zeros, or keep what they held, whatever is
+    in V. A NaN in q stays visible in its own row."""
+    q, k, v = (torch.randn(1, 64, 2, D, device="cuda").to(dtype) for _ in range(3))
+    v[:, 20] = bad
+    q[:, 60] = float("nan")
+    out, lse = _forward(q, k, v, True, -10)
+    assert (out[:, :10] == 0).all() and torch.isneginf(lse[:, :, :10]).all()
+    assert out[:, 60].isnan().all() and torch.isfinite(lse[:, :, 10:60]).all()
+    acc, old = torch.randn(1, 64, 2, D, device="cuda"), torch.randn(1, 2, 64, device="cuda")
+    acc2, lse2 = acc.clone(), old.clone()
+    _forward(q, k, v, True, -10, lse=lse2, out_acc=acc2, merge_prev=True)
+    assert torch.equal(acc2[:, :10], acc[:, :10]) and torch.equal(lse2[..., :10], old[..., :10])
