@@ -88,17 +88,18 @@ struct SimtShape {
   __device__ static __forceinline__ int col(int tx, int i) { return (i / kVec) * 64 + tx * kVec + i % kVec; }
 };
 
-// Cooperative load of kTile rows x D (element type T, row stride `stride` elements, rows >=
-// n_valid zero-filled) into an fp32 operand tile.
+// Cooperative load of kTile rows x D (element type T, row stride `stride` elements) into an fp32
+// operand tile; rows outside [first, end) are filled with zeros. The streamed operands are cut to
+// the rows that the block's own rows see or are seen by: a masked weight is 0, but 0 * Inf is not.
 template <int D, int R, typename T>
-__device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t stride, int n_valid) {
+__device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t stride, int end, int first = 0) {
   using S = SimtShape<D, R>;
   constexpr int kVecs = D / 4;
 #pragma unroll 4
   for (int i = threadIdx.x; i < kTile * kVecs; i += S::kThreads) {
     const int r = i / kVecs, f = i % kVecs;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < n_valid) v = load4<T>(src + (int64_t)r * stride + 4 * f);
+    if (r >= first && r < end) v = load4<T>(src + (int64_t)r * stride + 4 * f);
     *reinterpret_cast<float4*>(dst + r * S::kLd + 4 * f) = v;
   }
 }
@@ -260,8 +261,8 @@ attn_fwd_simt_kernel(const SimtFwdParams p) {
 
   for (int k0 = 0; k0 < n_keys; k0 += kTile) {
     __syncthreads();
-    load_tile<D, R, T>(k_s, kbase + (int64_t)k0 * p.k_ss, p.k_ss, p.Sk - k0);
-    load_tile<D, R, T>(v_s, vbase + (int64_t)k0 * p.v_ss, p.v_ss, p.Sk - k0);
+    load_tile<D, R, T>(k_s, kbase + (int64_t)k0 * p.k_ss, p.k_ss, n_keys - k0);
+    load_tile<D, R, T>(v_s, vbase + (int64_t)k0 * p.v_ss, p.v_ss, n_keys - k0);
     __syncthreads();
     float s[R][kCols], alpha[R];
     dot_tiles<D, R>(s, q_s, k_s, ty, tx);
@@ -418,8 +419,8 @@ attn_bwd_dq_simt_kernel(const SimtBwdParams p) {
 
   for (int k0 = 0; k0 < n_keys; k0 += kTile) {
     __syncthreads();
-    load_tile<D, R, T>(k_s, kbase + (int64_t)k0 * p.k_ss, p.k_ss, p.Sk - k0);
-    load_tile<D, R, T>(v_s, vbase + (int64_t)k0 * p.v_ss, p.v_ss, p.Sk - k0);
+    load_tile<D, R, T>(k_s, kbase + (int64_t)k0 * p.k_ss, p.k_ss, n_keys - k0);
+    load_tile<D, R, T>(v_s, vbase + (int64_t)k0 * p.v_ss, p.v_ss, n_keys - k0);
     __syncthreads();
     float s[R][kCols], dp[R][kCols];
     dot_tiles<D, R>(s, q_s, k_s, ty, tx);
@@ -494,25 +495,22 @@ attn_bwd_dkv_simt_kernel(const SimtBwdParams p) {
   for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int c = 0; c < S::kNC; ++c) dk[i][c] = dv[i][c] = 0.f;
-  int q_begin = 0;
-  if (p.causal) {
-    const long long first = (long long)r0 - p.causal_off;
-    q_begin = (int)max(0ll, min((long long)p.Sq, first));
-    q_begin = (q_begin / kTile) * kTile;
-  }
+  int q_first = 0;   // first query that sees a key of this block
+  if (p.causal) q_first = (int)max(0ll, min((long long)p.Sq, (long long)r0 - p.causal_off));
   for (int hh = 0; hh < G; ++hh) {
     const int h = g * G + hh;
     const T* qbase = reinterpret_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh;
     const T* dobase = reinterpret_cast<const T*>(p.dout) + b * p.do_sb + h * p.do_sh;
     const size_t sbase = (size_t)b * p.lse_sb + (size_t)h * p.lse_sh;
-    for (int q0 = q_begin; q0 < p.Sq; q0 += kTile) {
+    for (int q0 = q_first / kTile * kTile; q0 < p.Sq; q0 += kTile) {
       __syncthreads();
-      load_tile<D, R, T>(q_s, qbase + (int64_t)q0 * p.q_ss, p.q_ss, p.Sq - q0);
-      load_tile<D, R, T>(do_s, dobase + (int64_t)q0 * p.do_ss, p.do_ss, p.Sq - q0);
+      load_tile<D, R, T>(q_s, qbase + (int64_t)q0 * p.q_ss, p.q_ss, p.Sq - q0, q_first - q0);
+      load_tile<D, R, T>(do_s, dobase + (int64_t)q0 * p.do_ss, p.do_ss, p.Sq - q0, q_first - q0);
       if (threadIdx.x < kTile) {
         const int qi = q0 + threadIdx.x;
-        lse_s[threadIdx.x] = qi < p.Sq ? p.lse[sbase + qi] : INFINITY;
-        dl_s[threadIdx.x] = qi < p.Sq ? p.delta[sbase + qi] : 0.f;
+        const bool in = qi >= q_first && qi < p.Sq;
+        lse_s[threadIdx.x] = in ? p.lse[sbase + qi] : INFINITY;
+        dl_s[threadIdx.x] = in ? p.delta[sbase + qi] : 0.f;
       }
       __syncthreads();
       float s[R][kCols], dp[R][kCols];

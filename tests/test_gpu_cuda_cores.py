@@ -68,3 +68,35 @@ def test_rows_without_a_visible_key_ignore_the_values(D, dtype, bad):
     acc2, lse2 = acc.clone(), old.clone()
     _forward(q, k, v, True, -10, lse=lse2, out_acc=acc2, merge_prev=True)
     assert torch.equal(acc2[:, :10], acc[:, :10]) and torch.equal(lse2[..., :10], old[..., :10])
+
+
+@pytest.mark.parametrize("D,dtype", [(32, torch.float16), (64, torch.float32)])
+def test_keys_and_queries_outside_a_block_s_range_stay_outside(D, dtype):
+    """Infinities in keys that no query of a block sees, and in queries that see no key of a block,
+    leave the block's results as they are (the masked weight is 0, but 0 * Inf is not)."""
+    from sp_aurora_b200 import local_attn as la
+    inf = float("inf")
+
+    def grads(q, k, v, do, off):
+        out, lse = _forward(q, k, v, True, off)
+        dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
+        la.attn_bwd_step(q, k, v, do, lse, la.bwd_delta(out, do), D ** -0.5, True, None, dk, dv, causal_off=off,
+                         dq=dq, dq_overwrite=True)
+        return out, lse, dq, dk, dv
+    # 20 queries see the keys 0-19; key 40 is in the same tile
+    q, do = (torch.randn(1, 20, 2, D, device="cuda").to(dtype) for _ in range(2))
+    k, v = (torch.randn(1, 64, 2, D, device="cuda").to(dtype) for _ in range(2))
+    want = grads(q, k, v, do, 0)
+    k[:, 40], v[:, 40] = inf, inf
+    got = grads(q, k, v, do, 0)
+    for a, b in zip(got[:3], want[:3]):
+        assert torch.equal(a, b)
+    for a, b in zip(got[3:], want[3:]):
+        assert torch.equal(a[:, :40], b[:, :40]) and torch.equal(a[:, 41:], b[:, 41:])
+    # query i sees the keys up to i - 40: the keys from 64 on are seen from query 104 on
+    q, k, v, do = (torch.randn(1, 128, 2, D, device="cuda").to(dtype) for _ in range(4))
+    want = grads(q, k, v, do, -40)
+    do[:, 70], q[:, 80] = inf, inf
+    got = grads(q, k, v, do, -40)
+    for a, b in zip(got[3:], want[3:]):
+        assert torch.equal(a[:, 64:], b[:, 64:])
