@@ -105,21 +105,23 @@ __device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t stri
 }
 
 // acc[i][j] = row (ty + i*kTy) of a . row (tx + 16*j) of b. The even and the odd elements are
-// summed apart (the packed multiply-add works on pairs) and joined every 32 elements. Joined at the
-// end only, results were up to 14 % (D = 128) and 4 % (D = 64) further from 64-bit ones than those of
-// four threads per row; joining costs 2 % of the time (1127 -> 1151 us for the call above).
+// summed apart (the packed multiply-add works on pairs) and joined every 32 elements, at D = 32
+// every 16, so that no chain is longer than that of four threads per row, D / 4. Joined at the end
+// only, results were up to 14 % (D = 128), 4 % (D = 64) and 20 % (scores at D = 32) further from
+// 64-bit ones; joining costs 2 % of the time (1127 -> 1151 us for the call above).
 template <int D, int R>
 __device__ __forceinline__ void dot_tiles(float (&acc)[R][kCols], const float* a, const float* b, int ty, int tx) {
   using S = SimtShape<D, R>;
+  constexpr int kJoin = D == 32 ? 16 : 32;
 #pragma unroll
-  for (int f0 = 0; f0 < D; f0 += 32) {
+  for (int f0 = 0; f0 < D; f0 += kJoin) {
     float2 p[R][kCols];
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int j = 0; j < kCols; ++j) p[i][j] = make_float2(0.f, 0.f);
-#pragma unroll 2
-    for (int f = f0; f < f0 + 32; f += 4) {
+#pragma unroll(kJoin / 16)   // two steps at D = 32 spill
+    for (int f = f0; f < f0 + kJoin; f += 4) {
       float4 bv[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) bv[j] = *reinterpret_cast<const float4*>(b + (tx + 16 * j) * S::kLd + f);
