@@ -68,10 +68,10 @@ class SequenceParallelAttentionBlock(torch.nn.Module):
         hq, hkv = self.nheads, self.n_kv_heads
         qkv = self.qkv_proj(x).view(B, S, hq + 2 * hkv, self.head_dim)
         (cos, sin), offset = ((None, None), 0) if self.rope_base is None else self._rope_tables(S, x.device)
-        res = native.attention_heads_packed(qkv, hq, hkv, cos, sin, causal,
-                                            None if self.mode == "hybrid" else self.group)
-        if res is not None:      # one rank: rotation, attention and their gradients in one node
-            return self.out_proj(res[0].reshape(B, S, hq * self.head_dim))
+        if self.mode != "hybrid":    # there the submodule is called, with its hooks or what replaced it
+            res = native.attention_heads_packed(qkv, hq, hkv, cos, sin, causal, self.group)
+            if res is not None:      # one rank: rotation, attention and their gradients in one node
+                return self.out_proj(res[0].reshape(B, S, hq * self.head_dim))
         q, k, v = qkv[:, :, :hq], qkv[:, :, hq:hq + hkv], qkv[:, :, hq + hkv:]
         if self.rope_base is not None:
             qk = apply_rope(qkv[:, :, :hq + hkv], cos, sin, pos_offset=offset)   # one pass for q and k

@@ -194,3 +194,24 @@ def test_other_modes():
     y = q.clone().requires_grad_(True)
     h, = torch.autograd.grad(spa.ring_flash_attn_kvpacked_func(y, kv, causal=True), y, torch.ones_like(want))
     assert torch.equal(out, want) and torch.equal(g, h)
+
+
+@pytest.mark.parametrize("rope_base", [None, 10000.0])
+def test_hybrid_block_calls_its_submodule(rope_base):
+    """A forward hook on the block's attention module fires, and a module put in its place is used."""
+    import sp_aurora_b200 as spa
+    blk = spa.SequenceParallelAttentionBlock(512, 4, 2, mode="hybrid", device="cuda", rope_base=rope_base)
+    x, seen = _randn(1, 129, 512), []
+    handle = blk.hybrid.register_forward_hook(lambda mod, args, out: seen.append(out.shape))
+    y = blk(x)
+    assert seen == [(1, 129, 4, 128)]
+    handle.remove()
+    ring = spa.SequenceParallelAttentionBlock(512, 4, 2, mode="ring", device="cuda", rope_base=rope_base)
+    ring.load_state_dict(blk.state_dict())
+    assert torch.equal(ring(x), y)
+
+    class Zeros(torch.nn.Module):
+        def forward(self, q, k, v, causal):
+            return torch.zeros_like(q)
+    blk.hybrid = Zeros()
+    assert (blk(x) == 0).all()
