@@ -121,29 +121,32 @@ _SIGNATURES = {
 }
 
 
-def _rebuild_if_stale() -> str:
-    """Developer convenience: when a compiler is present and a source file is
-    newer than the library, recompile before loading (never a fallback: without
-    nvcc a stale or missing library still fails below). Returns the build error
-    text, if any, so that a missing library can be explained."""
+def _rebuild_if_stale():
+    """Developer convenience: when a compiler is present and a source file is newer than what was
+    built from it, recompile before loading (never a fallback: a missing file still fails below).
+    Returns the error if that failed, so that a missing or outdated file can be explained."""
     from . import build as _build   # plain build recipe, does not load the library
-    if os.environ.get("SPA_LIB_PATH"):
-        return ""
     try:
-        stale = _build._stale(_LIB_PATH, [_build.CSRC / s for s in _build.SOURCES] + _build.HEADERS)
-        if stale or _build._stale(_build.NATIVE_PATH, _build.NATIVE_DEPS):
-            _build.build()      # serialised across processes by a file lock; re-checks staleness
+        # SPA_LIB_PATH names another build of the library, which is taken as it is
+        cuda = not os.environ.get("SPA_LIB_PATH") and \
+            _build._stale(_LIB_PATH, [_build.CSRC / s for s in _build.SOURCES] + _build.HEADERS)
+        if cuda or _build._stale(_build.native_path(), _build.NATIVE_DEPS):
+            _build.build(cuda=cuda)      # serialised across processes by a file lock; re-checks staleness
     except RuntimeError as e:
-        return str(e)
-    return ""
+        return e
+    except OSError as e:
+        return _build.CannotBuild(str(e))
+    return None
+
+
+build_failure = _rebuild_if_stale()
 
 
 def _load() -> C.CDLL:
-    build_error = _rebuild_if_stale()
     if not _LIB_PATH.exists():
         raise ImportError(
             f"{_LIB_PATH} is missing: build it with `python sp_aurora_b200/build.py` "
-            "(this package has no fallback path)" + (f"\nlast build attempt:\n{build_error}" if build_error else ""))
+            "(this package has no fallback path)" + (f"\nlast build attempt:\n{build_failure}" if build_failure else ""))
     lib = C.CDLL(str(_LIB_PATH))
     for name, (res, args) in _SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError if the .so does not export it

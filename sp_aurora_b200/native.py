@@ -1,4 +1,4 @@
-"""One-rank attention through the C++ autograd node of `_native.so` (csrc/native_path.cpp).
+"""One-rank attention through the C++ autograd node of `_native-*.so` (csrc/native_path.cpp).
 
 Every function answers (out, lse), or None where the call has to go the general way: several
 ranks, per-kernel timing, or arguments that the node does not take (the general way also words
@@ -6,17 +6,31 @@ the errors)."""
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 
 import torch.distributed as dist
 
-from . import _lib, local_attn
+from . import _lib, build, local_attn
 
-try:
-    from . import _native
-except ImportError as e:
-    raise ImportError("_native.so is missing or was built against another torch: build it with "
-                      "`python sp_aurora_b200/build.py` (this package has no fallback path)") from e
 
+def _load(build_failure):
+    """The node built for this torch. One that is older than its sources is taken only where there
+    is no compiler to say whether it still fits: after a failed compilation it may read the
+    argument blocks of include/spa.h differently from the library."""
+    path = build.native_path()
+    outdated = path.exists() and build_failure is not None and \
+        not isinstance(build_failure, build.CannotBuild) and build._stale(path, build.NATIVE_DEPS)
+    if not path.exists() or outdated:
+        raise ImportError(f"{path} is {'older than its sources' if outdated else 'missing'}: build it with "
+                          "`python sp_aurora_b200/build.py` (this package has no fallback path)" +
+                          (f"\nlast build attempt:\n{build_failure}" if build_failure else ""))
+    spec = importlib.util.spec_from_file_location(f"{__package__}._native", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+_native = _load(_lib.build_failure)
 _native.set_api([C.cast(getattr(_lib.lib, name), C.c_void_p).value for name in (
     "spa_attn_fwd", "spa_attn_fwd_workspace", "spa_attn_fwd_ws", "spa_attn_bwd", "spa_attn_varlen_fwd",
     "spa_attn_varlen_bwd", "spa_bwd_delta", "spa_check_status", "spa_last_error", "spa_rope_rows")], _lib.SpaError)
