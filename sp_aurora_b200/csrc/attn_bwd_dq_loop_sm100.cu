@@ -569,21 +569,32 @@ int launch_dq_loop_any(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
             : launch_dq_loop_typed<64, __half, kVar>(a, 0, seqs, n_seq);
 }
 
+// K/V tiles that the `blocks` query tiles of a sequence go through all together.
+long long walk_tiles(long long blocks, int sk, bool causal, int causal_off) {
+  const long long n = ceil_div(sk, kTileN);
+  if (!causal) return blocks * n;
+  // Tile i (the last one taken as full) sees first + i K/V tiles, cut to 0..n.
+  const long long last_key = kTileM - 1 + (long long)causal_off;   // of tile 0
+  const long long first = last_key >= 0 ? last_key / kTileN + 1 : -((-last_key - 1) / kTileN);
+  auto sum_to = [](long long x) { return x > 0 ? x * (x + 1) / 2 : 0ll; };
+  return sum_to(first + blocks - 1) - sum_to(first - 1) - sum_to(first + blocks - 1 - n) + sum_to(first - 1 - n);
+}
+
 }  // namespace
 
-// Several items for every SM and short walks: at most 24 K/V tiles on average (measured: 12 tiles
-// 251 -> 224 us, 16 tiles 241 -> 222, 32 tiles even; beyond that a fixed schedule loses, its CTAs
-// drift apart and stop sharing K/V in L2: 32768 rows 11.8 -> 14.3 ms).
+// Several items for every SM and short walks: at most 24 K/V tiles on average without a mask, or 48
+// query tiles that start at the diagonal (24.5). Measured: 12 tiles 251 -> 224 us, 16 tiles 241 ->
+// 222, 32 tiles even; beyond that a fixed schedule loses, its CTAs drift apart and stop sharing K/V
+// in L2: 32768 rows 11.8 -> 14.3 ms.
 bool dq_loops(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
   if (a->D != 64 && a->D != 128) return false;
   long long items = 0, walk = 0;
   for (int i = 0; i < (n_seq > 0 ? n_seq : 1); ++i) {
     const long long blocks = ceil_div(n_seq > 0 ? seqs[i].sq : a->Sq, kTileM);
     items += blocks;
-    walk += blocks * ceil_div(n_seq > 0 ? seqs[i].sk : a->Sk, kTileN);
+    walk += walk_tiles(blocks, n_seq > 0 ? seqs[i].sk : a->Sk, a->causal, n_seq > 0 ? seqs[i].causal_off : a->causal_off);
   }
-  if (a->causal) walk /= 2;
-  return items * a->Hq * a->B >= 3ll * device_sm_count() && walk <= 24 * items;
+  return items * a->Hq * a->B >= 3ll * device_sm_count() && 2 * walk <= 49 * items;
 }
 
 int launch_bwd_dq_loop_sm100(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
