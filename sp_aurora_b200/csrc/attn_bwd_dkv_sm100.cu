@@ -534,9 +534,14 @@ attn_bwd_dkv_sm100_kernel(const __grid_constant__ CUtensorMap tm_q,
         load_cols(which == 0 ? t_dv : t_dk, which == 0 ? 1.f : p.scale, o);
         if (!key_ok) continue;
         T* drow = reinterpret_cast<T*>(which == 0 ? p.dv : p.dk) + row_off;
-        if (p.dkv_accumulate) {
+        if (p.dkv_accumulate) {   // past the L1, as the row statistics
 #pragma unroll
-          for (int i = 0; i < kCols; ++i) o[i] += static_cast<float>(drow[i]);
+          for (int i = 0; i < kCols / 8; ++i) {
+            const uint4 u = __ldcg(reinterpret_cast<const uint4*>(drow) + i);
+            const T* old = reinterpret_cast<const T*>(&u);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[8 * i + j] += static_cast<float>(old[j]);
+          }
         }
         uint4* dst = reinterpret_cast<uint4*>(drow);
 #pragma unroll

@@ -57,3 +57,29 @@ def test_loop_over_packed_sequences():
         for x, y in zip((out[:, hq], lse[hq], dq[:, hq], dk[:, hk], dv[:, hk]), (o, l, *g)):
             assert torch.equal(x, y), h
     spa.check_status()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_gradients_added_to_16_bit_tensors_beside_the_dq_pass(D):
+    """Both passes in one call, 13 key tiles (the dK/dV pass starts beside the dQ pass), dK/dV added
+    to element-type tensors: the fp32 gradient plus the old row, rounded once."""
+    import sp_aurora_b200 as spa
+    from sp_aurora_b200 import local_attn as la
+    B, S, H, Hk = 1, 1600, 4, 2
+    q, do = (torch.randn(B, S, H, D, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, S, Hk, D, device="cuda").bfloat16() for _ in range(2))
+    out, lse = spa.flash_attn_forward(q, k, v, None, True)
+    delta = la.bwd_delta(out, do)
+    dk32, dv32 = (torch.empty(B, S, Hk, D, device="cuda") for _ in range(2))
+    dq = torch.empty_like(q)
+    la.attn_bwd_step(q, k, v, do, lse, delta, D ** -0.5, True, None, dk32, dv32, dq=dq, dq_overwrite=True,
+                     deterministic=True)
+    old = torch.randn(B, S, 2, Hk, D, device="cuda").bfloat16()
+    dkv = torch.empty_like(old)
+    for _ in range(3):                      # the tensors are written again just before each call
+        dkv.copy_(old)
+        la.attn_bwd_step(q, k, v, do, lse, delta, D ** -0.5, True, None, dkv[:, :, 0], dkv[:, :, 1],
+                         dkv_accumulate=True, dq=dq, dq_overwrite=True)
+        assert torch.equal(dkv[:, :, 0], (dk32 + old[:, :, 0].float()).bfloat16())
+        assert torch.equal(dkv[:, :, 1], (dv32 + old[:, :, 1].float()).bfloat16())
+    spa.check_status()
