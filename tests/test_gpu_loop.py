@@ -83,3 +83,36 @@ def test_gradients_added_to_16_bit_tensors_beside_the_dq_pass(D):
         assert torch.equal(dkv[:, :, 0], (dk32 + old[:, :, 0].float()).bfloat16())
         assert torch.equal(dkv[:, :, 1], (dv32 + old[:, :, 1].float()).bfloat16())
     spa.check_status()
+
+
+@pytest.mark.parametrize("off", [0, -300])       # -300: query tiles without a visible key
+@pytest.mark.parametrize("overwrite", [False, True])
+@pytest.mark.parametrize("with_dq", [False, True])
+def test_loop_over_a_running_sum(off, overwrite, with_dq):
+    """A ring step's form of the dQ pass (fp32 sum in and out): bitwise the calls on one batch
+    entry, which have too few query tiles to loop."""
+    import sp_aurora_b200 as spa
+    from sp_aurora_b200 import _lib, local_attn as la
+    B, Sq, Sk, H, Hk, D = 5, 900, 700, 32, 4, 128
+    g = torch.Generator(device="cuda").manual_seed(13)
+    q, do = (torch.randn(B, Sq, H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Sk, Hk, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    acc0 = torch.randn(B, Sq, H, D, device="cuda", generator=g)
+    out, lse = torch.empty_like(q), torch.empty(B, H, Sq, device="cuda")
+    la.attn_fwd_step(q, k, v, D ** -0.5, True, lse, out=out, causal_off=off)
+    delta = la.bwd_delta(out, do)
+
+    def call(sl):
+        acc = acc0[sl].clone()
+        dq = torch.zeros_like(q[sl]) if with_dq else None
+        la.attn_bwd_step(q[sl], k[sl], v[sl], do[sl], lse[sl], delta[sl], D ** -0.5, True, acc, None, None,
+                         causal_off=off, dq=dq, dq_overwrite=overwrite, passes=_lib.SPA_BWD_DQ_ONLY)
+        return acc, dq
+    acc, dq = call(slice(0, B))
+    for b in range(B):
+        a, d = call(slice(b, b + 1))
+        assert torch.equal(acc[b:b + 1], a), b
+        assert d is None or torch.equal(dq[b:b + 1], d), b
+    spa.check_status()
+    if off and not overwrite:
+        assert torch.equal(acc[:, :300], acc0[:, :300])      # rows that see nothing keep their sum

@@ -9,9 +9,15 @@ def _randn(*shape, dtype=torch.bfloat16):
     return torch.randn(*shape, device="cuda", dtype=dtype)
 
 
-def _grads(fn, leaves, dout):
+def _is_node(t):
+    """t came out of the C++ node and not of a Python autograd function."""
+    return "CppNode" in t.grad_fn.name()
+
+
+def _grads(fn, leaves, dout, node):
     leaves = [t.detach().clone().requires_grad_(True) for t in leaves]
     out, lse, _ = fn(*leaves)
+    assert _is_node(out) == node, out.grad_fn.name()
     return [out.detach(), lse.detach(), *torch.autograd.grad(out, leaves, dout)]
 
 
@@ -58,9 +64,9 @@ def test_same_results_as_the_python_functions(general, kind, dtype, D):
               "qkv": spa.ring_flash_attn_qkvpacked_func, "ulysses": spa.ulysses_flash_attn_func,
               "zigzag": spa.zigzag_ring_flash_attn_func}[kind]
         fn = (lambda f: lambda *x: f(*x, **kw))(fn)
-    a = _grads(fn, leaves, do)
+    a = _grads(fn, leaves, do, node=True)
     with general():
-        b = _grads(fn, leaves, do)
+        b = _grads(fn, leaves, do, node=False)
     spa.check_status()
     for x, y in zip(a, b):
         assert x.shape == y.shape and torch.equal(x, y)
@@ -71,6 +77,7 @@ def test_node_behaves_like_an_autograd_function():
     backward needs retain_graph, an in-place change of an input is noticed."""
     import sp_aurora_b200 as spa
     q, k, v = (_randn(1, 130, 2, 64).requires_grad_(True) for _ in range(3))
+    assert _is_node(spa.select_flash_attn_impl()(q, k, v))
     packed = []
     with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or t.cpu(), lambda t: t.cuda()):
         out = spa.ring_flash_attn_func(q, k, v, causal=True)
@@ -150,7 +157,7 @@ def test_forward_and_backward_are_captured_in_a_graph(S):
 
 @pytest.mark.parametrize("mode", ["ring", "ulysses"])
 @pytest.mark.parametrize("rope_base", [None, 10000.0])
-def test_block_node_equals_the_sliced_form(general, mode, rope_base):
+def test_block_node_equals_the_sliced_form(general, monkeypatch, mode, rope_base):
     """Rotation, attention and the joined gradient of one projection output. Bitwise: adding the
     zeros of the other slices changes nothing, the rotation is undone from the same 16-bit rows."""
     import sp_aurora_b200 as spa
@@ -162,9 +169,13 @@ def test_block_node_equals_the_sliced_form(general, mode, rope_base):
         t = x.clone().requires_grad_(True)
         y = blk(t, causal=True)
         return [y.detach(), *torch.autograd.grad(y, (t, *blk.parameters()), dy)]
+    from sp_aurora_b200 import native
+    taken, call = [], native.attention_heads_packed
+    monkeypatch.setattr(native, "attention_heads_packed", lambda *x: taken.append(call(*x)) or taken[-1])
     a = step()
     with general():
         b = step()
+    assert taken[0] is not None and taken[1] is None     # the node, then the sliced form
     spa.check_status()
     for p, q in zip(a, b):
         assert torch.equal(p, q)

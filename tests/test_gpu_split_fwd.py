@@ -29,13 +29,19 @@ def _needed(q, k, v, causal):
 
 
 @pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,D,dtype,causal,split", [
-    (1, 1, 2049, 4, 2, 128, torch.bfloat16, False, True),       # one row, a ragged last tile
-    (2, 128, 4096, 8, 2, 128, torch.bfloat16, False, True),     # one tile, heads paired
-    (1, 129, 2500, 8, 8, 64, torch.float16, False, True),       # two tiles, one row in the second
-    (1, 300, 3000, 4, 2, 64, torch.bfloat16, False, True),      # three tiles: pairs of heads
-    (1, 3000, 3000, 4, 2, 128, torch.bfloat16, True, True),     # causal: early slices of early rows are empty
-    (1, 640, 640, 4, 2, 128, torch.float16, True, False),       # pairs, too few keys to split
-    (3, 130, 900, 6, 2, 64, torch.float16, False, False),       # odd group: no pairing
+    # one query tile per CTA (a CTA per tile fits the chip)
+    (1, 1, 2049, 4, 2, 128, torch.bfloat16, False, True),       # one row, a ragged last key tile
+    (2, 128, 4096, 8, 2, 128, torch.bfloat16, False, True),
+    (1, 129, 2500, 8, 8, 64, torch.float16, False, True),       # one row in the second query tile
+    (1, 300, 3000, 4, 2, 64, torch.bfloat16, False, True),
+    (1, 3000, 3000, 4, 2, 128, torch.bfloat16, True, True),     # two tiles per CTA; early slices of early rows are empty
+    (1, 640, 640, 4, 2, 128, torch.float16, True, False),       # too few keys to split
+    (3, 130, 900, 6, 2, 64, torch.float16, False, False),
+    # odd tile counts: heads paired
+    (3, 300, 2100, 16, 8, 64, torch.bfloat16, False, True),     # and the keys split
+    (2, 100, 1500, 32, 8, 128, torch.float16, False, True),
+    (16, 640, 640, 4, 2, 128, torch.bfloat16, True, False),
+    (26, 300, 300, 6, 2, 64, torch.float16, False, False),      # odd group: no pairing
 ])
 def test_short_grids_match_the_oracle(B, Sq, Sk, Hq, Hkv, D, dtype, causal, split):
     import sp_aurora_b200 as spa
@@ -86,3 +92,30 @@ def test_workspace_size_is_checked():
     torch.cuda.synchronize()
     assert (lse - lse2).abs().max() < 1e-5
     assert (out.float() - out2.float()).abs().max() <= 2 ** -7 * out.float().abs().max()
+
+
+@pytest.mark.parametrize("Sq,D,causal,off", [(300, 128, True, 40), (257, 64, False, 0), (640, 64, True, -200)])
+def test_head_pairs_merge_into_a_running_result(Sq, D, causal, off):
+    """A ring step's form (fp32 result and lse in and out) on grids whose CTAs take one query tile
+    of two heads: bitwise the calls on one head, which has no partner (odd tile counts, 2 query
+    heads per kv head, more tiles than SMs, so neither the split nor single tiles apply)."""
+    import sp_aurora_b200 as spa
+    from sp_aurora_b200 import local_attn as la
+    B, Sk, Hq, Hkv = 25, 500, 4, 2
+    g = torch.Generator(device="cuda").manual_seed(17)
+    q = torch.randn(B, Sq, Hq, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(B, Sk, Hkv, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    acc0, lse0 = torch.randn(B, Sq, Hq, D, device="cuda"), torch.randn(B, Hq, Sq, device="cuda")
+
+    def call(hq, hk):
+        acc, lse = acc0[:, :, hq].clone(), lse0[:, hq].clone()
+        out = torch.empty_like(q[:, :, hq])
+        la.attn_fwd_step(q[:, :, hq], k[:, :, hk], v[:, :, hk], D ** -0.5, causal, lse, out=out, out_acc=acc,
+                         merge_prev=True, causal_off=off)
+        return acc, lse, out
+    acc, lse, out = call(slice(0, Hq), slice(0, Hkv))
+    for h in range(Hq):
+        a, l, o = call(slice(h, h + 1), slice(h // 2, h // 2 + 1))
+        assert torch.equal(acc[:, :, h:h + 1], a) and torch.equal(lse[:, h:h + 1], l), h
+        assert torch.equal(out[:, :, h:h + 1], o), h
+    spa.check_status()
