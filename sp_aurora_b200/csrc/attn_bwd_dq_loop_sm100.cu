@@ -592,7 +592,8 @@ bool dq_loops(const spa_bwd_args* a, const spa_seq* seqs, int n_seq) {
   for (int i = 0; i < (n_seq > 0 ? n_seq : 1); ++i) {
     const long long blocks = ceil_div(n_seq > 0 ? seqs[i].sq : a->Sq, kTileM);
     items += blocks;
-    walk += walk_tiles(blocks, n_seq > 0 ? seqs[i].sk : a->Sk, a->causal, n_seq > 0 ? seqs[i].causal_off : a->causal_off);
+    walk += n_seq > 0 ? walk_tiles(blocks, seqs[i].sk, a->causal, seqs[i].causal_off)
+                      : walk_tiles(blocks, a->Sk, a->causal, a->causal_off);
   }
   return items * a->Hq * a->B >= 3ll * device_sm_count() && 2 * walk <= 49 * items;
 }

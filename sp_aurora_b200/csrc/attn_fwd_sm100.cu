@@ -563,6 +563,17 @@ struct FwdPlan {
 // through a key tile in 0.7 of the time that two need in turn, and there are SMs to spare (512
 // rows of 4 heads 18.5 -> 16.4 us, 2 x 1024 rows of 8 heads 24.6 -> 22.5).
 // Times are in units of one key tile of two query tiles (2.2 us).
+// Where the lines lie, and what lies beyond them (us):
+// - pairing for odd counts up to 5 tiles: 1, 3, 5 tiles over 2048 keys 138 -> 82, 148 -> 119, 220 ->
+//   192 (batch 16, 8, 8 of 32 / 8 heads), causal 3 and 5 tiles 43 -> 35, 79 -> 67. Longer odd counts
+//   stay with the plain instance; most would gain as well (9 tiles 189 -> 158, 13 causal 76 -> 65,
+//   7 tiles 151 either way).
+// - at least 4 key tiles a slice, so that a slice fills its pipeline: with 8 instead 15 -> 21 (128
+//   queries of 4 heads over 2048 keys); with 2 even there and better below (1024 keys 19 -> 12).
+// - at most 16 slices, which bounds the workspace: with 8 instead 27 -> 37 (1 query of 4 heads over
+//   16384 keys); with 32 better from there on with few heads (27 -> 23, 131072 keys 138 -> 81).
+// - a finer plan has to promise 7 % more, for what the model leaves out: over 40 drawn calls the times
+//   lie 1.2 % above the best margin of each call, with 0, 3 and 12 % 1.1, 0.3 and 4.4 %.
 FwdPlan plan_fwd(const spa_fwd_args* a, bool workspace) {
   FwdPlan plan{false, false, 1};
   const int tiles = ceil_div(a->Sq, kTileM);

@@ -13,8 +13,9 @@
 // the next product's operand go through shared memory rows that only their own warp reads (no
 // block barrier). Tile rows are padded by four floats, which puts the 16 rows a half-warp reads
 // at once in different banks. B=2, S=1024, 32 heads, D=64, causal, fp32: forward + backward
-// 2486 -> 1151 us against four threads per row with one float4 load per four multiply-adds;
-// the three kernels now run at 29, 35 and 35 TFLOP/s executed of the 73 an FMA-only loop reaches.
+// 2486 -> 1154 us against four threads per row with one float4 load per four multiply-adds; the
+// three kernels take 293, 368 and 496 us, 31, 37 and 37 TFLOP/s of executed tiles of the 73 that an
+// FMA-only loop reaches.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math.h>
@@ -108,7 +109,8 @@ __device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t stri
 // summed apart (the packed multiply-add works on pairs) and joined every 32 elements, at D = 32
 // every 16, so that no chain is longer than that of four threads per row, D / 4. Joined at the end
 // only, results were up to 14 % (D = 128), 4 % (D = 64) and 20 % (scores at D = 32) further from
-// 64-bit ones; joining costs 2 % of the time (1127 -> 1151 us for the call above).
+// 64-bit ones; joining costs 2 % of the time (1127 -> 1151 us for the call above), at D = 32 up to 7 %
+// (1024 rows of 2 x 8 heads 309 -> 322 us, 3000 of 8 in bf16 927 -> 990, 3000 of 32 2725 -> 2703).
 template <int D, int R>
 __device__ __forceinline__ void dot_tiles(float (&acc)[R][kCols], const float* a, const float* b, int ty, int tx) {
   using S = SimtShape<D, R>;
@@ -120,7 +122,7 @@ __device__ __forceinline__ void dot_tiles(float (&acc)[R][kCols], const float* a
     for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int j = 0; j < kCols; ++j) p[i][j] = make_float2(0.f, 0.f);
-#pragma unroll(kJoin / 16)   // two steps at D = 32 spill
+#pragma unroll(kJoin / 16)   // two steps at D = 32 spill: 322 -> 324, 990 -> 954, 2703 -> 2773 us
     for (int f = f0; f < f0 + kJoin; f += 4) {
       float4 bv[kCols];
 #pragma unroll
@@ -609,8 +611,9 @@ int launch_simt(void (*kern)(P), const P& p, int operand_tiles, int extra_floats
   return SPA_OK;
 }
 
-// Rows per thread: 8 load less per multiply-add, but at D = 128 the accumulators of 8 rows spill
-// (S=2900, 8 heads: dK/dV 2825 us with 8, 2196 with 4; S=1024, 32 heads, D = 64: 479 and 502).
+// Rows per thread: 8 load less per multiply-add. At D = 64 they are faster although the backward
+// kernels spill 40 (dK/dV) and 88 bytes (dQ) at 255 registers (S=1024, 32 heads: dK/dV 479 us with 8,
+// 502 with 4); at D = 128 the accumulators of 8 rows spill far more (S=2900, 8 heads: 2825 and 2196).
 template <int D>
 constexpr int kSimtR = D == 128 ? 4 : 8;
 

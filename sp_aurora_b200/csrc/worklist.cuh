@@ -5,20 +5,21 @@
 // that takes several items keeps its copies and products running across them.
 //
 // The items come longest first; CTA c takes one from each run of gridDim.x, alternately from the
-// run's front and its back, which gives every CTA the same mix (within 1 % of longest-first
-// dispatch by the hardware for 3000 to 32768 causal rows of 32 heads). The threads of a CTA decode
-// its items side by side into shared memory at the start; the warps read them from there.
+// run's front and its back, which gives every CTA nearly the same number of tiles (within 1 % of
+// what longest-first dispatch by the hardware gives, for 3000 to 32768 causal rows of 32 heads). In
+// time that holds for short walks only: in long ones the CTAs drift apart (see dq_loops). The
+// threads of a CTA decode its items side by side into shared memory at the start; the warps read
+// them from there.
 #pragma once
 #include <stdint.h>
 
 namespace spa {
 
 struct alignas(16) WorkItem {
-  int h, b;          // head, batch
-  int r0;            // first row of the stationary tile in its sequence
-  int sg, part;      // sequence of a packed batch, slice of a split item
-  int n0, n1;        // tiles of the streamed operand (for the first / second stationary tile)
-  int base;          // first row of the slice
+  int h, b;   // head, batch
+  int r0;     // first row of the stationary tile in its sequence
+  int sg;     // sequence of a packed batch
+  int n0;     // tiles of the streamed operand
 };
 
 __device__ __forceinline__ int item_index(int pos) {
